@@ -2082,7 +2082,7 @@ void moe_sort(const Tensor& chosen, Tensor& order, Tensor& offsets) {
 }
 
 void moe_gate_up(const Tensor& x, const Tensor& w, const Tensor& order, const Tensor& offsets, Tensor& act, int64_t top,
-                 double limit, double slope, int64_t form, double up_offset) {
+                 double limit, double slope, int64_t form, double up_offset, const OptTensor& status) {
   check_cuda(x, "x");
   check_cuda(w, "w");
   check_cuda(act, "act");
@@ -2110,15 +2110,16 @@ void moe_gate_up(const Tensor& x, const Tensor& w, const Tensor& order, const Te
   p.slope = (float)slope;
   p.up_offset = (float)up_offset;
   p.dtype = dtype_code(x, "x");
-  AKV_CHECK(form >= 0 && form <= 3, "form: 0 by size, 1 float arithmetic, 2 mma.sync tiles, 3 few rows");
+  AKV_CHECK(form >= 0 && form <= 4, "form: 0 by size, 1 float arithmetic, 2 mma.sync tiles, 3 few rows, 4 tcgen05 tiles");
   p.force_plain = (int)form;
+  p.status = status_ptr(status);
   c10::cuda::CUDAGuard guard(x.device());
   check_launch(akv::launch_moe_gemm(p, akv::kMoeGated, stream_of(x)), "moe_gate_up");
 }
 
 // act[r] = activation(w[expert of sorted row r] x[token of that row]): experts without a gate.
 void moe_up(const Tensor& x, const Tensor& w, const Tensor& order, const Tensor& offsets, Tensor& act, int64_t top,
-            int64_t activation, int64_t form) {
+            int64_t activation, int64_t form, const OptTensor& status) {
   check_cuda(x, "x");
   check_cuda(w, "w");
   check_cuda(act, "act");
@@ -2131,7 +2132,7 @@ void moe_up(const Tensor& x, const Tensor& w, const Tensor& order, const Tensor&
   AKV_CHECK(top >= 1 && pairs == x.size(0) * top && act.numel() == pairs * inter,
             "moe_up: order holds tokens * top pairs, act [pairs, intermediate]");
   AKV_CHECK(activation >= 0 && activation <= akv::kActLast, "moe_up: unknown activation");
-  AKV_CHECK(form >= 0 && form <= 3, "form: 0 by size, 1 float arithmetic, 2 mma.sync tiles, 3 few rows");
+  AKV_CHECK(form >= 0 && form <= 4, "form: 0 by size, 1 float arithmetic, 2 mma.sync tiles, 3 few rows, 4 tcgen05 tiles");
   akv::MoeGemmParams p{};
   p.a = x.data_ptr();
   p.w = w.data_ptr();
@@ -2146,12 +2147,13 @@ void moe_up(const Tensor& x, const Tensor& w, const Tensor& order, const Tensor&
   p.activation = (int)activation;
   p.dtype = dtype_code(x, "x");
   p.force_plain = (int)form;
+  p.status = status_ptr(status);
   c10::cuda::CUDAGuard guard(x.device());
   check_launch(akv::launch_moe_gemm(p, akv::kMoeUp, stream_of(x)), "moe_up");
 }
 
 void moe_down(const Tensor& act, const Tensor& w, const Tensor& order, const Tensor& offsets, const Tensor& weights,
-              Tensor& out, int64_t form) {
+              Tensor& out, int64_t form, const OptTensor& status) {
   check_cuda(act, "act");
   check_cuda(w, "w");
   check_same(act, w, "act", "w");
@@ -2175,8 +2177,9 @@ void moe_down(const Tensor& act, const Tensor& w, const Tensor& order, const Ten
   p.n = (int)hidden;
   p.top = 1;
   p.dtype = dtype_code(act, "act");
-  AKV_CHECK(form >= 0 && form <= 3, "form: 0 by size, 1 float arithmetic, 2 mma.sync tiles, 3 few rows");
+  AKV_CHECK(form >= 0 && form <= 4, "form: 0 by size, 1 float arithmetic, 2 mma.sync tiles, 3 few rows, 4 tcgen05 tiles");
   p.force_plain = (int)form;
+  p.status = status_ptr(status);
   c10::cuda::CUDAGuard guard(act.device());
   check_launch(akv::launch_moe_gemm(p, akv::kMoeDown, stream_of(act)), "moe_down");
 }
@@ -2394,11 +2397,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("moe_router", &moe_router, py::arg("x"), py::arg("w"), py::arg("logits"));
   m.def("moe_sort", &moe_sort, py::arg("chosen"), py::arg("order"), py::arg("offsets"));
   m.def("moe_gate_up", &moe_gate_up, py::arg("x"), py::arg("w"), py::arg("order"), py::arg("offsets"), py::arg("act"),
-        py::arg("top"), py::arg("limit"), py::arg("slope"), py::arg("form") = 0, py::arg("up_offset") = 1.0);
+        py::arg("top"), py::arg("limit"), py::arg("slope"), py::arg("form") = 0, py::arg("up_offset") = 1.0,
+        py::arg("status") = py::none());
   m.def("moe_up", &moe_up, py::arg("x"), py::arg("w"), py::arg("order"), py::arg("offsets"), py::arg("act"),
-        py::arg("top"), py::arg("activation"), py::arg("form") = 0);
+        py::arg("top"), py::arg("activation"), py::arg("form") = 0, py::arg("status") = py::none());
   m.def("moe_down", &moe_down, py::arg("act"), py::arg("w"), py::arg("order"), py::arg("offsets"), py::arg("weights"),
-        py::arg("out"), py::arg("form") = 0);
+        py::arg("out"), py::arg("form") = 0, py::arg("status") = py::none());
   m.def("moe_combine", &moe_combine, py::arg("parts"), py::arg("shared"), py::arg("out"), py::arg("top"),
         py::arg("chosen") = py::none(), py::arg("pair_weights") = py::none(), py::arg("x") = py::none(),
         py::arg("first_identity") = 0);

@@ -422,13 +422,18 @@ struct MoeGemmParams {
   float limit, slope;
   float up_offset;             // the gated product's activation is g sigmoid(slope g) (u + up_offset)
   int dtype;
-  int force_plain;             // 0: the form is chosen by size; 1: float arithmetic; 2: mma.sync tiles; 3: few rows
+  int force_plain;             // 0: the form is chosen by size; 1: float arithmetic; 2: mma.sync tiles; 3: few rows;
+                               // 4: tcgen05 tiles (routed_experts_tc.cu)
   int activation;              // up: an Activation
+  int* status;                 // kernels' status word, or null
 };
-// steps with at most this many (token, choice) pairs run the few-rows form of the gated product (measured at 8
-// tokens, 64 experts of 1,024 x 4,096: 103 against 111 us; the down product is faster in tiles: 59 against 89 us)
+// steps with at most this many (token, choice) pairs that the tcgen05 form does not take run the few-rows form of the
+// gated product (against mma.sync tiles at 8 tokens, 64 experts of 1,024 x 4,096: 103 against 111 us; the down product
+// is faster in tiles: 59 against 89 us)
 constexpr int kMoeFewRowPairs = 128;
 int launch_moe_gemm(const MoeGemmParams& p, MoeForm form, cudaStream_t stream);
+bool moe_gemm_takes_tc(const MoeGemmParams& p, MoeForm form);
+int launch_moe_gemm_tc(const MoeGemmParams& p, MoeForm form, cudaStream_t stream);
 // out[t] = sum over c < top of parts[t * top + c] (+ shared[t]), float32; with `chosen` the choices from
 // first_identity on count as pair_weights[t, c] * x[t].
 int launch_moe_combine(const float* parts, const void* shared, int shared_dtype, float* out, int64_t num_tokens,

@@ -425,11 +425,10 @@ __device__ __forceinline__ void find_tile_of(const int32_t* offsets, int experts
 }
 }  // namespace
 
-template <int FORM, int BM>
+template <int FORM>
 __global__ void __launch_bounds__(256) moe_gemm_mma_kernel(MoeGemmParams p) {
   constexpr bool GATED = FORM == kMoeGated, FIRST = FORM != kMoeDown;
-  // BM sorted rows of one expert per CTA (64, or 128 where experts have rows enough to fill such tiles: a warp then
-  // holds 64 x 32 of the output and every weight fragment it fetches serves four row fragments instead of two)
+  constexpr int BM = kMmaRows;                      // sorted rows of one expert per CTA
   extern __shared__ __align__(16) unsigned char mma_smem[];
   typedef __nv_bfloat16 (*ATile)[BM][kMmaPitch];
   typedef __nv_bfloat16 (*WTile)[kMmaWeightRows][kMmaPitch];
@@ -586,14 +585,15 @@ static bool moe_gemm_takes_mma(const MoeGemmParams& p) {
          (reinterpret_cast<uintptr_t>(p.a) | reinterpret_cast<uintptr_t>(p.w)) % 16 == 0;
 }
 
-template <int FORM, int BM>
+template <int FORM>
 static int launch_moe_mma(const MoeGemmParams& p, cudaStream_t stream) {
+  constexpr int BM = kMmaRows;
   const int64_t row_tiles = p.pairs / BM + (p.pairs < p.experts ? p.pairs : p.experts);
   const int cols = FORM == kMoeGated ? kMmaWeightRows / 2 : kMmaWeightRows;
   const int64_t col_tiles = (p.n + cols - 1) / cols;
   if (row_tiles > 65535 || col_tiles > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
   const size_t smem = sizeof(__nv_bfloat16) * kMmaStages * (BM + kMmaWeightRows) * kMmaPitch;
-  auto kernel = moe_gemm_mma_kernel<FORM, BM>;
+  auto kernel = moe_gemm_mma_kernel<FORM>;
   if (smem > 48 * 1024) {
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return (int)err;
@@ -707,8 +707,14 @@ __global__ void __launch_bounds__(kGemvWarps * 32) moe_gemv_kernel(MoeGemmParams
 namespace {
 template <int FORM>
 int launch_moe_form(const MoeGemmParams& p, cudaStream_t stream) {
-  // 0: by size; 1: float arithmetic; 2: mma.sync tiles; 3: the few-rows form
+  // 0: by size; 1: float arithmetic; 2: mma.sync tiles; 3: the few-rows form; 4: tcgen05 tiles.  Whatever the tcgen05
+  // form takes it is the fastest at every size measured (us, gated / down product, 64 experts of 1,024 x 4,096 with 6
+  // choices, tcgen05 | mma.sync tiles | few rows): 1 token 43 / 22 | 81 / 33 | 62 / 29; 8 tokens 103 / 55 | 123 / 68 |
+  // 115 / 68; 64 tokens 195 / 109 | 275 / 143 | 470 / 224; 2,048 tokens 282 / 185 | 881 / 520.  The other two serve
+  // hidden sizes below one K block of 64.
   const bool tensor_ok = moe_gemm_takes_mma(p);
+  if (p.force_plain == 4 || (p.force_plain == 0 && moe_gemm_takes_tc(p, (MoeForm)FORM)))
+    return launch_moe_gemm_tc(p, (MoeForm)FORM, stream);
   if ((p.force_plain == 2 || p.force_plain == 3) && !tensor_ok) return (int)cudaErrorInvalidValue;
   if (p.force_plain == 3 || (p.force_plain == 0 && tensor_ok && FORM != kMoeDown && p.pairs <= kMoeFewRowPairs)) {
     const int64_t col_tiles = (p.n + kGemvFeatures - 1) / kGemvFeatures;
@@ -716,16 +722,7 @@ int launch_moe_form(const MoeGemmParams& p, cudaStream_t stream) {
     const dim3 grid((unsigned)col_tiles, (unsigned)p.experts);
     return (int)launch_chain(moe_gemv_kernel<FORM>, grid, dim3(kGemvWarps * 32), 0, stream, dim3(1, 1, 1), p);
   }
-  if (tensor_ok && p.force_plain != 1) {
-    // tiles of 128 rows where the experts' runs are long enough to fill them.  Measured (gated / down product, us):
-    // 256 rows an expert 244 / 142 against 234 / 138 with tiles of 64; 128 rows 669 / 388 against 652 / 371; 512 rows
-    // 1,937 / 1,203 against 2,141 / 1,268.  AKV_MOE_TALL_ROWS moves the threshold (a measurement switch).
-    static const int64_t tall_rows = [] {
-      const char* v = getenv("AKV_MOE_TALL_ROWS");
-      return v != nullptr && v[0] != '\0' ? (int64_t)atoll(v) : (int64_t)384;
-    }();
-    return p.pairs >= tall_rows * p.experts ? launch_moe_mma<FORM, 128>(p, stream) : launch_moe_mma<FORM, 64>(p, stream);
-  }
+  if (tensor_ok && p.force_plain != 1) return launch_moe_mma<FORM>(p, stream);
   // every expert may end in a tile that is not full
   const int64_t row_tiles = p.pairs / kTileRows + (p.pairs < p.experts ? p.pairs : p.experts);
   const int64_t col_tiles = (p.n + kTileCols - 1) / kTileCols;

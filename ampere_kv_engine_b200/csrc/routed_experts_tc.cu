@@ -1,0 +1,361 @@
+// The routed experts' grouped products on the 5th-generation tensor cores (bfloat16): for the sorted rows of every
+// expert,   out[r, f] = sum_k w[expert, f, k] * a[row(r), k]
+// with the activation (first products) or the pair's weight (down product) on the output tile.
+//
+// The weights are the M operand, 256 rows per CTA as two tcgen05.mma tiles of 128 (gated: 128 gate rows and the 128 up
+// rows of the same features, so that a thread of the epilogue holds a feature's both halves); the rows of ONE expert,
+// up to 256 of them, are the N operand, N being their number rounded up to 16.  So an expert's matrix leaves HBM once
+// whatever its number of rows, which is the bound from a handful of rows to a few hundred an expert, and an expert's
+// rows are read by a CTA for 256 weight rows at a time: at 150 rows an expert a K block of 64 moves 32 KB of weights
+// and 19 KB of rows from the L2 (with 128 weight rows per CTA it would be 16 and 19).  The weights come by TMA, the rows
+// by cp.async from where they lie (no pass that sorts them first): TMA gathers of four rows take 50 ns each, 596 us
+// for the first product below where cp.async took 330.
+//
+// Persistent: one CTA per SM takes tiles blockIdx, blockIdx + grid, ...  Warp 0 copies weights into a ring of 3 to 6
+// stages (as many as fit beside the widest tile of the launch), warps 2-5 the rows, warp 1 issues the MMAs, warps 6-13
+// drain the two accumulators (256 of the 512 TMEM columns each).  A tile is drained before the next one's MMAs begin; the ring fills meanwhile, and
+// the next tile's first stages are there when the drain ends.  Within an expert neighbouring CTAs take the row tiles of
+// one weight tile, so that a second row tile finds the weights in the L2.
+//
+// Measured (us, first / second product, L2 flushed; the mma.sync form before): 12,288 rows over 64 experts of 1,024 x
+// 4,096 282 / 185 (881 / 520), 8,192 rows over 32 experts of 768 x 2,048 100 / 70 (241 / 143), 128 rows over the 64
+// experts 187 / 101 (270 / 134; the few-rows form 249 / 136).  The weights alone take 164 / 82 us at the copy bandwidth;
+// what keeps a prompt from it is the ring: at 200 rows a stage is 57 KB, three fit, and the memory's latency is not
+// covered (DRAM at 39 %, the tensor pipe and the crossbar far below their limits).
+//
+// Every wait is bounded; a wait that runs out sets kWaitTimeout in the status word, copies under way are waited for,
+// and the CTA frees its TMEM and leaves.
+#include "common.cuh"
+#include "launchers.h"
+#include "tcgen05.cuh"
+#include "tensor_map.h"
+
+namespace akv {
+
+namespace {
+
+constexpr int kK = 64;                        // K elements per stage: 128 bytes, one swizzle row
+constexpr int kMaxRows = 256;                 // rows of an expert per tile
+constexpr int kHalf = 128;                    // weight rows per MMA
+constexpr int kWeightBytes = 2 * kHalf * kK * 2;
+constexpr int kRing = 216 * 1024;             // the stages' shared memory
+constexpr int kMaxStages = 6;
+constexpr int kRowWarps = 4;
+constexpr int kEpilogueWarps = 8;
+constexpr int kThreads = 32 * (2 + kRowWarps + kEpilogueWarps);
+
+struct Shared {
+  uint64_t full[kMaxStages], empty[kMaxStages], acc_full, acc_empty;
+  uint32_t tmem;
+  int widest;                                 // rows of the widest tile
+  int failed;
+  int tile_start[kMoeMaxExperts + 1];         // row tiles before each expert
+};
+constexpr int kSmemBytes = 1024 + kRing + (int)sizeof(Shared);
+
+__device__ __forceinline__ int round16(int n) { return (n + 15) & ~15; }
+// rows of each of an expert's tiles (the last one may have fewer): balanced, a multiple of 16
+__device__ __forceinline__ int tile_rows_of(int count, int tiles) { return min(kMaxRows, round16((count + tiles - 1) / tiles)); }
+
+struct Tile {
+  int expert, m, row0, rows;
+};
+// Tiles are numbered expert by expert, within an expert weight tile by weight tile, row tiles fastest.
+__device__ __forceinline__ Tile tile_of(const Shared& s, const int32_t* offsets, int experts, int m_tiles, int tile) {
+  const int q = tile / m_tiles;
+  int low = 0, high = experts;                // the last expert whose first tile is not behind q
+  while (high - low > 1) {
+    const int mid = (low + high) >> 1;
+    if (s.tile_start[mid] <= q) low = mid;
+    else high = mid;
+  }
+  const int begin = offsets[low], count = offsets[low + 1] - begin;
+  const int tiles = s.tile_start[low + 1] - s.tile_start[low], local = tile - s.tile_start[low] * m_tiles;
+  const int per = tile_rows_of(count, tiles);
+  Tile t;
+  t.expert = low;
+  t.m = local / tiles;
+  t.row0 = begin + (local - t.m * tiles) * per;
+  t.rows = min(per, begin + count - t.row0);
+  return t;
+}
+
+__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, bool inside) {
+  const int bytes = inside ? 16 : 0;          // zero bytes read: the 16 bytes are filled with zeros
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+}  // namespace
+
+template <int FORM>
+__global__ void __launch_bounds__(kThreads, 1)
+moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, MoeGemmParams p) {
+  constexpr bool GATED = FORM == kMoeGated, FIRST = FORM != kMoeDown;
+  constexpr int kFeatures = GATED ? kHalf : 2 * kHalf;          // output features per tile
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  Shared& s = *reinterpret_cast<Shared*>(ring + kRing);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  pdl_launch_dependents();
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kMaxStages; ++i) {
+      tc::mbar_init(&s.full[i], 1 + kRowWarps);
+      tc::mbar_init(&s.empty[i], 1);
+    }
+    tc::mbar_init(&s.acc_full, 1);
+    tc::mbar_init(&s.acc_empty, kEpilogueWarps);
+    s.failed = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) tc::tmem_alloc(&s.tmem, 512);
+  pdl_wait();
+  if (warp == 0) {
+    // row tiles before each expert, and the widest tile
+    int before = 0, widest = 0;
+    for (int e0 = 0; e0 < p.experts; e0 += 32) {
+      const int e = e0 + lane;
+      const int count = e < p.experts ? p.offsets[e + 1] - p.offsets[e] : 0;
+      const int tiles = (count + kMaxRows - 1) / kMaxRows;
+      if (tiles > 0) widest = max(widest, tile_rows_of(count, tiles));
+      int sum = tiles;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += v;
+      }
+      if (e < p.experts) s.tile_start[e] = before + sum - tiles;
+      before += __shfl_sync(0xffffffffu, sum, 31);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) widest = max(widest, __shfl_xor_sync(0xffffffffu, widest, o));
+    if (lane == 0) {
+      s.tile_start[p.experts] = before;
+      s.widest = widest;
+    }
+  }
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  const uint32_t tmem = s.tmem;
+  const int m_tiles = (p.n + kFeatures - 1) / kFeatures;
+  const int tiles = s.tile_start[p.experts] * m_tiles;
+  const int stage_bytes = kWeightBytes + s.widest * kK * 2;
+  const int stages = min(kMaxStages, kRing / stage_bytes);
+  const int blocks = (p.k + kK - 1) / kK;
+  bool ok = true;
+  int stage = 0, issued = 0;
+  uint32_t phase = 0;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+        const Tile t = tile_of(s, p.offsets, p.experts, m_tiles, tile);
+        const int w_row = t.expert * (GATED ? 2 : 1) * p.n + t.m * kFeatures;
+        for (int kb = 0; kb < blocks; ++kb) {
+          if (!tc::mbar_wait(&s.empty[stage], phase ^ 1)) {
+            ok = false;
+            break;
+          }
+          uint8_t* at = ring + stage * stage_bytes;
+          tc::mbar_expect_tx(&s.full[stage], (uint32_t)kWeightBytes);
+          tc::tma_load_2d(at, &w_map, kb * kK, w_row, &s.full[stage]);
+          tc::tma_load_2d(at + kWeightBytes / 2, &w_map, kb * kK, w_row + (GATED ? p.n : kHalf), &s.full[stage]);
+          ++issued;
+          if (++stage == stages) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+      }
+    }
+  } else if (warp >= 2 && warp < 2 + kRowWarps) {
+    // Rows r0, r0 + 16, ... of the tile, 16-byte piece `piece` of each K block: 128-byte rows with the 128-byte swizzle
+    // (piece c of row r at c ^ (r & 7)).  Rows beyond the tile's repeat its last one, their results unused.
+    const int id = (warp - 2) * 32 + lane, piece = id & 7, r0 = id >> 3;
+    const uint32_t place = tc::smem_u32(ring) + kWeightBytes + r0 * (kK * 2) + ((piece ^ (r0 & 7)) << 4);
+    const __nv_bfloat16* a = (const __nv_bfloat16*)p.a;
+    int signalled = 0;          // the next stage whose rows are to be announced
+    auto announce = [&] {
+      // the tensor core reads through the async proxy: this thread's finished copies are made visible to it first
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&s.full[signalled]);
+      if (++signalled == stages) signalled = 0;
+    };
+    // Copies of U stages are left under way.  The rows of block b are announced after those of block b + U were issued,
+    // which waits until block b + U - stages has been multiplied: with U = stages - 1 every product would wait for the
+    // one before it and for the copies issued in between (12,288 rows, first product: 330 us against 282).
+    const int most = stages >= 5 ? 3 : stages - 2;
+    int under_way = 0;
+    for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+      const Tile t = tile_of(s, p.offsets, p.experts, m_tiles, tile);
+      int source[kMaxRows / 16];
+#pragma unroll
+      for (int i = 0; i < kMaxRows / 16; ++i) {
+        const int r = t.row0 + min(r0 + 16 * i, t.rows - 1);
+        source[i] = 16 * i < t.rows ? (FIRST ? p.order[r] / p.top : r) : 0;
+      }
+      for (int kb = 0; kb < blocks; ++kb) {
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(&s.empty[stage], phase ^ 1));
+        if (!ok) break;
+        const int k = kb * kK + piece * 8;
+        const bool inside = k < p.k;
+        const uint32_t dst = place + stage * stage_bytes;
+#pragma unroll
+        for (int i = 0; i < kMaxRows / 16; ++i)
+          if (16 * i < t.rows)
+            cp_async_16(dst + i * 16 * kK * 2, a + (inside ? (int64_t)source[i] * p.k + k : 0), inside);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (++under_way > most) {
+          if (most == 1) cp_async_wait<1>();
+          else if (most == 2) cp_async_wait<2>();
+          else cp_async_wait<3>();
+          announce();
+          --under_way;
+        }
+        if (++stage == stages) {
+          stage = 0;
+          phase ^= 1;
+        }
+      }
+    }
+    cp_async_wait<0>();
+    for (; under_way > 0; --under_way) announce();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int done = 0;
+      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++done) {
+        const uint32_t idesc = tc::umma_idesc(round16(tile_of(s, p.offsets, p.experts, m_tiles, tile).rows));
+        if (done > 0 && !tc::mbar_wait(&s.acc_empty, (uint32_t)(done - 1) & 1u)) {
+          ok = false;
+          break;
+        }
+        tc::fence_after();
+        for (int kb = 0; kb < blocks; ++kb) {
+          if (!tc::mbar_wait(&s.full[stage], phase)) {
+            ok = false;
+            break;
+          }
+          tc::fence_after();
+          const uint32_t w_addr = tc::smem_u32(ring + stage * stage_bytes), a_addr = w_addr + kWeightBytes;
+#pragma unroll
+          for (int k = 0; k < kK / 16; ++k) {
+            // 16 K elements = 32 bytes further along the swizzled row
+            const uint32_t more = (kb > 0 || k > 0) ? 1u : 0u;
+            const uint64_t rows_desc = tc::umma_desc(a_addr + k * 32);
+            tc::umma_bf16(tmem, tc::umma_desc(w_addr + k * 32), rows_desc, idesc, more);
+            tc::umma_bf16(tmem + kMaxRows, tc::umma_desc(w_addr + kWeightBytes / 2 + k * 32), rows_desc, idesc, more);
+          }
+          tc::umma_commit(&s.empty[stage]);
+          if (++stage == stages) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+        if (ok) tc::umma_commit(&s.acc_full);
+      }
+    }
+  } else {
+    // a lane is one feature of each half, a column one row; the two groups of four warps take columns in turn
+    const int quarter = warp & 3, group = (warp - 2 - kRowWarps) >> 2;
+    const uint32_t lanes = tmem + ((uint32_t)(quarter * 32) << 16);
+    int done = 0;
+    for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++done) {
+      const Tile t = tile_of(s, p.offsets, p.experts, m_tiles, tile);
+      const int feature = t.m * kFeatures + quarter * 32 + lane;
+      ok = __all_sync(0xffffffffu, tc::mbar_wait(&s.acc_full, (uint32_t)done & 1u));
+      if (!ok) break;
+      tc::fence_after();
+#pragma unroll 1
+      for (int c = group * 16; c < t.rows; c += 32) {
+        uint32_t first[16], second[16];
+        tc::tmem_load16(lanes + c, first);
+        tc::tmem_load16(lanes + kMaxRows + c, second);
+        int pair = 0;
+        float weight = 0.f;
+        if constexpr (!FIRST) {
+          // lanes 0-15 fetch the pair and the weight of one row each
+          if (lane < 16 && c + lane < t.rows) {
+            pair = p.order[t.row0 + c + lane];
+            weight = p.weights[pair];
+          }
+        }
+        tc::tmem_wait_load();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          if (c + j >= t.rows) break;
+          const float x = __uint_as_float(first[j]), y = __uint_as_float(second[j]);
+          if constexpr (GATED) {
+            const float g = fminf(x, p.limit);
+            const float u = fminf(fmaxf(y, -p.limit), p.limit);
+            if (feature < p.n)
+              ((__nv_bfloat16*)p.out)[(int64_t)(t.row0 + c + j) * p.n + feature] =
+                  __float2bfloat16_rn(g / (1.f + expf(-p.slope * g)) * (u + p.up_offset));
+          } else if constexpr (FIRST) {
+            __nv_bfloat16* dst = (__nv_bfloat16*)p.out + (int64_t)(t.row0 + c + j) * p.n + feature;
+            if (feature < p.n) dst[0] = __float2bfloat16_rn(activation_value(x, p.activation));
+            if (feature + kHalf < p.n) dst[kHalf] = __float2bfloat16_rn(activation_value(y, p.activation));
+          } else {
+            const float w = __shfl_sync(0xffffffffu, weight, j);
+            float* dst = (float*)p.out + (int64_t)__shfl_sync(0xffffffffu, pair, j) * p.n + feature;
+            if (feature < p.n) dst[0] = w * x;
+            if (feature + kHalf < p.n) dst[kHalf] = w * y;
+          }
+        }
+      }
+      tc::fence_before();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&s.acc_empty);
+    }
+  }
+  if (!ok) {
+    set_status(p.status, kWaitTimeout);
+    s.failed = 1;
+  }
+  tc::fence_before();
+  __syncthreads();
+  if (s.failed && threadIdx.x == 0) {
+    // weights under way that nobody waits for any more: time to land before the shared memory goes
+    for (int i = max(0, issued - stages); i < issued; ++i) tc::mbar_wait(&s.full[i % stages], (uint32_t)(i / stages) & 1u);
+  }
+  if (warp == 1) tc::tmem_free(tmem, 512);
+}
+
+bool moe_gemm_takes_tc(const MoeGemmParams& p, MoeForm form) {
+  const int64_t weight_rows = (int64_t)p.experts * (form == kMoeGated ? 2 : 1) * p.n;
+  return p.dtype == kBFloat16 && p.k % 8 == 0 && p.k >= kK && weight_rows <= 0x7fffffffLL && p.pairs <= 0x7fffffffLL &&
+         (reinterpret_cast<uintptr_t>(p.a) | reinterpret_cast<uintptr_t>(p.w)) % 16 == 0;
+}
+
+template <int FORM>
+static int launch_form(const MoeGemmParams& p, cudaStream_t stream) {
+  constexpr int kFeatures = FORM == kMoeGated ? kHalf : 2 * kHalf;
+  CUtensorMap w_map;
+  if (!weight_tensor_map(p.w, (int64_t)p.experts * (FORM == kMoeGated ? 2 : 1) * p.n, p.k, kHalf, &w_map))
+    return (int)cudaErrorInvalidValue;
+  const int64_t row_tiles = p.pairs / kMaxRows + (p.pairs < p.experts ? p.pairs : p.experts);     // at most
+  const int64_t tiles = row_tiles * ((p.n + kFeatures - 1) / kFeatures);
+  if (tiles > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
+  auto kernel = moe_gemm_tc_kernel<FORM>;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    if (err != cudaSuccess) return (int)err;
+    configured = true;
+  }
+  const int64_t grid = tiles < sm_count() ? tiles : sm_count();
+  return (int)launch_chain(kernel, dim3((unsigned)grid), dim3(kThreads), kSmemBytes, stream, dim3(1, 1, 1), w_map, p);
+}
+
+int launch_moe_gemm_tc(const MoeGemmParams& p, MoeForm form, cudaStream_t stream) {
+  if (!moe_gemm_takes_tc(p, form)) return (int)cudaErrorInvalidValue;
+  switch (form) {
+    case kMoeGated: return launch_form<kMoeGated>(p, stream);
+    case kMoeUp: return launch_form<kMoeUp>(p, stream);
+    default: return launch_form<kMoeDown>(p, stream);
+  }
+}
+
+}  // namespace akv

@@ -617,7 +617,7 @@ def delta_scan(qkv, coef, x, norm_weight, state, cu_q, state_slots, *, num_heads
 
 MOE_MAX_EXPERTS = 512
 MOE_MAX_TOP = 32
-MOE_FORMS = {"auto": 0, "plain": 1, "mma": 2, "few": 3}
+MOE_FORMS = {"auto": 0, "plain": 1, "mma": 2, "few": 3, "tc": 4}
 
 
 #: steps of at most this many tokens compute the router's logits with a warp per (token, expert); the library's
@@ -665,38 +665,44 @@ def moe_sort(chosen, experts: int):
     return order, offsets
 
 
-def moe_gate_up(x, w_gate_up, order, offsets, *, top, limit, slope, kernel: str = "auto", up_offset: float = 1.0):
+def _status_of(status, x) -> dict:
+    """The kernels' status word, for the grouped products that have bounded waits (they run on the GPU alone)."""
+    return {"status": status} if status is not None and x.is_cuda else {}
+
+
+def moe_gate_up(x, w_gate_up, order, offsets, *, top, limit, slope, kernel: str = "auto", up_offset: float = 1.0,
+                status=None):
     """Row r of the result belongs to pair ``order[r]`` and is its expert's ``g * sigmoid(slope * g) * (u + up_offset)``
     with ``g = min(W_gate x, limit)``, ``u = clamp(W_up x, -limit, limit)`` for the pair's token (an infinite limit, a
     slope of one and no offset make it ``silu(g) * u``);
     ``w_gate_up`` [experts, gate rows then up rows, hidden].  [tokens * top, intermediate] in the dtype of ``x``.
-    ``kernel``: ``"auto"``: for bfloat16 with a hidden size that is a multiple of eight, the few-rows form (weights
-    streamed once, no staging) for the gated product of steps of up to 128 pairs and the tensor cores (``mma.sync``
-    tiles) otherwise;
-    ``"plain"`` keeps the float-arithmetic form, which is also all of float32; ``"mma"`` / ``"few"`` force one."""
+    ``kernel``: ``"auto"``: for bfloat16 with a hidden size that is a multiple of eight and at least 64 the tcgen05 tiles
+    (below 64 ``mma.sync`` tiles or, for the gated product of up to 128 pairs, the few-rows form);
+    ``"plain"`` keeps the float-arithmetic form, which is also all of float32; ``"tc"`` / ``"mma"`` / ``"few"`` force one."""
     inter = w_gate_up.shape[1] // 2
     act = torch.empty((order.numel(), inter), dtype=x.dtype, device=x.device)
     ext().moe_gate_up(x, w_gate_up, order, offsets, act, top, float(limit), float(slope), MOE_FORMS[kernel],
-                      float(up_offset))
+                      float(up_offset), **_status_of(status, x))
     _launched()
     return act
 
 
-def moe_up(x, w_up, order, offsets, *, top, activation: str, kernel: str = "auto"):
+def moe_up(x, w_up, order, offsets, *, top, activation: str, kernel: str = "auto", status=None):
     """Row r of the result belongs to pair ``order[r]`` and is ``activation(W_up x)`` of its expert (one without a gate)
     for the pair's token; ``w_up`` [experts, intermediate, hidden].  [tokens * top, intermediate] in the dtype of ``x``.
     ``kernel`` as for :func:`moe_gate_up`."""
     act = torch.empty((order.numel(), w_up.shape[1]), dtype=x.dtype, device=x.device)
-    ext().moe_up(x, w_up, order, offsets, act, top, ACTIVATIONS[activation], MOE_FORMS[kernel])
+    ext().moe_up(x, w_up, order, offsets, act, top, ACTIVATIONS[activation], MOE_FORMS[kernel],
+                 **_status_of(status, x))
     _launched()
     return act
 
 
-def moe_down(act, w_down, order, offsets, weights, kernel: str = "auto"):
+def moe_down(act, w_down, order, offsets, weights, kernel: str = "auto", status=None):
     """``weights[pair] * W_down[expert] act[r]`` for every sorted row r, written to row ``order[r]`` of a float32
     [tokens * top, hidden].  ``kernel`` as for :func:`moe_gate_up`."""
     out = torch.empty((order.numel(), w_down.shape[1]), dtype=torch.float32, device=act.device)
-    ext().moe_down(act, w_down, order, offsets, weights, out, MOE_FORMS[kernel])
+    ext().moe_down(act, w_down, order, offsets, weights, out, MOE_FORMS[kernel], **_status_of(status, act))
     _launched()
     return out
 

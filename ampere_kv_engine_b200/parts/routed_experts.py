@@ -147,10 +147,11 @@ class RoutedExperts(FeedForward):
             offsets = offsets[:self.experts + 1]       # the identity choices' pairs sort behind the experts' runs
         if self.gated:
             act = ops.moe_gate_up(x, self.w_gate_up, order, offsets, top=self.top, limit=self.limit,
-                                  slope=self.swish_slope, up_offset=self.up_offset)
+                                  slope=self.swish_slope, up_offset=self.up_offset, status=status)
         else:
-            act = ops.moe_up(x, self.w_gate_up, order, offsets, top=self.top, activation=self.activation)
-        parts = ops.moe_down(act, self.w_down, order, offsets, weights)
+            act = ops.moe_up(x, self.w_gate_up, order, offsets, top=self.top, activation=self.activation,
+                             status=status)
+        parts = ops.moe_down(act, self.w_down, order, offsets, weights, status=status)
         shared = None
         if self.shared_size:
             if self.activation == "silu":

@@ -1,0 +1,87 @@
+"""The routed experts' products on tcgen05 tiles: runs at the edges of the row tiles (1, 16, 17, 256, 257, 513 rows of
+one expert, an expert without rows), K and feature counts that end inside a block or a tile, choices that are no
+expert's."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(counts, k, n, top, form, seed=0):
+    """Tokens whose first choice gives expert e ``counts[e]`` rows; further choices beyond the experts (identity)."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    tokens, experts = sum(counts), len(counts)
+    first = torch.repeat_interleave(torch.arange(experts, device="cuda"), torch.tensor(counts, device="cuda"))
+    chosen = torch.full((tokens, top), experts, dtype=torch.int32, device="cuda")
+    chosen[:, top - 1] = first[torch.randperm(tokens, generator=g, device="cuda")].int()
+    x = torch.randn(tokens, k, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(experts, (2 if form == "gated" else 1) * n, k, generator=g, device="cuda") * k ** -0.5).bfloat16()
+    return x, w, chosen, torch.rand(tokens, top, generator=g, device="cuda") + 0.5
+
+
+@pytest.mark.parametrize("form", ["gated", "up", "down"])
+@pytest.mark.parametrize("counts,k,n", [([1, 0, 3], 64, 1), ([16, 17, 1], 72, 130), ([256, 0, 257], 200, 128),
+                                        ([513, 40], 136, 257), ([5000], 64, 40)])
+def test_products_at_the_edges_of_the_tiles(form, counts, k, n):
+    from ampere_kv_engine_b200.kernels import ops
+
+    top, experts = 2, len(counts)
+    x, w, chosen, weights = _case(counts, k, n, top, form)
+    order, offsets = ops.moe_sort(chosen, experts + 1)
+    offsets = offsets[:experts + 1]
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    rows = int(offsets[-1])
+    assert rows == sum(counts)
+    source = order[:rows].long() // top
+    expert = torch.repeat_interleave(torch.arange(experts, device="cuda"), offsets.diff().long())
+    wide = w.double()
+    if form == "down":
+        act = torch.zeros(order.numel(), k, dtype=torch.bfloat16, device="cuda")
+        act[:rows] = x[source]
+        got = ops.moe_down(act, w, order, offsets, weights, kernel="tc", status=status)[order[:rows].long()].double()
+        scale = weights.view(-1)[order[:rows].long()][:, None].double()
+    else:
+        scale = 1.0
+    want, size = torch.empty(rows, n, dtype=torch.float64, device="cuda"), None
+    size = torch.empty_like(want)
+    for e in range(experts):
+        at = expert == e
+        a = x[source[at]].double()
+        z, bound = a @ wide[e].T, a.abs() @ wide[e].abs().T
+        if form == "gated":
+            gate, up = z[:, :n].clamp(max=2.0), z[:, n:].clamp(-2.0, 2.0)
+            want[at] = gate * torch.sigmoid(1.702 * gate) * (up + 1.0)
+            # |d act / d gate| <= 1.2 |up + 1| <= 3.6, |d act / d up| <= |gate| <= max(2, |z|)
+            size[at] = 3.6 * bound[:, :n] + bound[:, n:] * z[:, :n].abs().clamp(min=2.0)
+        elif form == "up":
+            want[at], size[at] = torch.relu(z).square(), 2.0 * z.abs() * bound
+        else:
+            want[at], size[at] = z, bound
+    if form == "gated":
+        got = ops.moe_gate_up(x, w, order, offsets, top=top, limit=2.0, slope=1.702, kernel="tc", status=status)
+        got = got[:rows].double()
+    elif form == "up":
+        got = ops.moe_up(x, w, order, offsets, top=top, activation="relu2", kernel="tc", status=status)[:rows].double()
+    # k products added up in float32 (each addition off by at most 2^-24 of the sums' size, twice that if truncated), the
+    # approximations of a float32 exponential and division, then one rounding to bfloat16 (down: to float32)
+    stored = 0.0 if form == "down" else 2.0 ** -8
+    assert int(status) == 0
+    error = (got - scale * want).abs()
+    assert bool((error <= scale * (k * 2.0 ** -23 * size + 2.0 ** -21 * want.abs()) + stored * want.abs() + 1e-30).all())
+
+
+def test_a_row_is_the_same_whatever_shares_its_tile():
+    from ampere_kv_engine_b200.kernels import ops
+
+    x, w, chosen, _ = _case([300, 20], 256, 96, 1, "gated", seed=3)
+
+    def rows(first, stop):
+        """The products of these tokens, in the tokens' order (the order within an expert's run is any)."""
+        order, offsets = ops.moe_sort(chosen[first:stop].contiguous(), 2)
+        act = ops.moe_gate_up(x[first:stop].contiguous(), w, order, offsets, top=1, limit=7.0, slope=1.702, kernel="tc")
+        return torch.empty_like(act).index_copy_(0, order.long(), act)
+
+    everyone = rows(0, 320)
+    for t in (0, 150, 319):
+        assert torch.equal(rows(t, t + 1)[0], everyone[t])
