@@ -820,6 +820,93 @@ void scored_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_ca
   check_launch(akv::launch_scored_attention(sp, stream_of(q)), "scored_attention");
 }
 
+// out[r] = the cache row of the plan's r-th key, zeros behind a sequence's context (launchers.h describes the plan).
+void latent_gather(const Tensor& cache, const Tensor& block_table, const Tensor& plan, Tensor& out, int64_t num_seqs,
+                   const OptTensor& status) {
+  check_cuda(cache, "cache");
+  check_cuda(out, "out");
+  check_same(cache, out, "cache", "out");
+  AKV_CHECK(cache.scalar_type() == at::kBFloat16 && cache.dim() == 4 && cache.size(1) == 1 && out.dim() == 2 &&
+                out.size(1) == cache.size(3) && cache.size(3) % 8 == 0,
+            "latent_gather: bfloat16 cache [pages, 1, page size, width], out [rows, width], a width of whole 16-byte pieces");
+  check_i32(block_table, "block_table");
+  AKV_CHECK(block_table.dim() == 2, "block_table must be [sequences, width]");
+  check_i32(plan, "plan");
+  AKV_CHECK(num_seqs >= 1 && plan.numel() >= num_seqs * akv::kLatentPlanSeq, "latent_gather: the plan is too short");
+  akv::LatentGatherParams p{};
+  p.cache = cache.data_ptr();
+  p.block_table = block_table.data_ptr<int>();
+  p.plan = plan.data_ptr<int>();
+  p.out = out.data_ptr();
+  p.rows = out.size(0);
+  p.num_pages = cache.size(0);
+  p.num_seqs = (int)num_seqs;
+  p.page_size = (int)cache.size(2);
+  p.table_width = (int)block_table.size(1);
+  p.width = (int)cache.size(3);
+  p.status = status_ptr(status);
+  c10::cuda::CUDAGuard guard(cache.device());
+  check_launch(akv::launch_latent_gather(p, stream_of(cache)), "latent_gather");
+}
+
+void latent_prompt_attention(const Tensor& q, const Tensor& q_rows, const Tensor& kv, const Tensor& latents, Tensor& out,
+                             const Tensor& plan, int64_t num_seqs, int64_t num_tiles, int64_t heads, int64_t dim,
+                             int64_t rot_dim, int64_t v_dim, int64_t rank, int64_t window, double scale,
+                             const OptTensor& gate, const OptTensor& sink, const OptTensor& status) {
+  AKV_CHECK(q.is_cuda() && q.dim() == 2 && q.stride(1) == 1 && q.size(1) >= heads * (dim + rot_dim) &&
+                reinterpret_cast<uintptr_t>(q.data_ptr()) % 16 == 0,
+            "latent_prompt_attention: q [tokens, heads * (dim + rot_dim) and more], rows contiguous, 16-byte aligned");
+  check_cuda(q_rows, "q_rows");
+  check_cuda(kv, "kv");
+  check_cuda(latents, "latents");
+  check_cuda(out, "out");
+  check_same(kv, q_rows, "kv", "q_rows");
+  check_same(kv, latents, "kv", "latents");
+  check_same(kv, out, "kv", "out");
+  AKV_CHECK(q.scalar_type() == at::kBFloat16 && kv.scalar_type() == at::kBFloat16 && q.device() == kv.device(),
+            "latent_prompt_attention: bfloat16 on one device");
+  const int64_t n = q.size(0), rows = latents.size(0);
+  AKV_CHECK(heads >= 1 && akv::latent_prompt_supported((int)dim, (int)rot_dim, (int)v_dim, (int)rank) && window >= 0 && scale > 0,
+            "latent_prompt_attention: widths outside what the kernel takes");
+  AKV_CHECK(q_rows.numel() == n * heads * (rank + rot_dim) && latents.dim() == 2 && latents.size(1) == rank + rot_dim &&
+                kv.numel() == rows * heads * (dim + v_dim) && out.numel() == n * heads * v_dim && rows % 128 == 0,
+            "latent_prompt_attention: q_rows [tokens, heads, rank + rot_dim], latents [rows, rank + rot_dim], kv [rows, "
+            "heads, dim + v_dim], out [tokens, heads, v_dim], rows a multiple of 128");
+  check_i32(plan, "plan");
+  AKV_CHECK(num_seqs >= 1 && num_tiles >= 0 && plan.numel() >= num_seqs * akv::kLatentPlanSeq + 2 * num_tiles,
+            "latent_prompt_attention: the plan is too short");
+  akv::LatentPromptParams p{};
+  if (gate.has_value()) {
+    check_f32(*gate, "gate", n * heads);
+    p.gate = gate->data_ptr<float>();
+  }
+  if (sink.has_value()) {
+    check_f32(*sink, "sink", heads);
+    p.sink = sink->data_ptr<float>();
+  }
+  p.q = q.data_ptr();
+  p.q_rows = q_rows.data_ptr();
+  p.kv = kv.data_ptr();
+  p.latents = latents.data_ptr();
+  p.out = out.data_ptr();
+  p.plan = plan.data_ptr<int>();
+  p.num_tokens = n;
+  p.rows = rows;
+  p.q_stride = q.stride(0);
+  p.num_seqs = (int)num_seqs;
+  p.num_tiles = (int)num_tiles;
+  p.heads = (int)heads;
+  p.dim = (int)dim;
+  p.rot_dim = (int)rot_dim;
+  p.v_dim = (int)v_dim;
+  p.rank = (int)rank;
+  p.window = (int)window;
+  p.scale = (float)scale;
+  p.status = status_ptr(status);
+  c10::cuda::CUDAGuard guard(kv.device());
+  check_launch(akv::launch_latent_prompt(p, stream_of(kv)), "latent_prompt_attention");
+}
+
 void head_prep(const Tensor& x, const OptTensor& slots, Tensor& q_out, const OptTensor& k_cache,
                const OptTensor& v_cache, const OptTensor& v_keep, const OptTensor& v_other,
                const OptTensor& blend_weight, const OptTensor& gate_out, int64_t num_heads, int64_t num_kv_heads,
@@ -2391,6 +2478,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("token_gate", &token_gate, py::arg("z"), py::arg("ids"), py::arg("sampled"), py::arg("table"), py::arg("col_off"),
         py::arg("out"), py::arg("status") = py::none());
   m.def("scaled_sum", &scaled_sum, py::arg("a"), py::arg("b"), py::arg("out"), py::arg("sa"), py::arg("sb"));
+  m.def("latent_gather", &latent_gather, py::arg("cache"), py::arg("block_table"), py::arg("plan"), py::arg("out"),
+        py::arg("num_seqs"), py::arg("status") = py::none());
+  m.def("latent_prompt_attention", &latent_prompt_attention, py::arg("q"), py::arg("q_rows"), py::arg("kv"),
+        py::arg("latents"), py::arg("out"), py::arg("plan"), py::arg("num_seqs"), py::arg("num_tiles"), py::arg("heads"),
+        py::arg("dim"), py::arg("rot_dim"), py::arg("v_dim"), py::arg("rank"), py::arg("window"), py::arg("scale"),
+        py::arg("gate") = py::none(), py::arg("sink") = py::none(), py::arg("status") = py::none());
   m.def("moe_route", &moe_route, py::arg("logits"), py::arg("correction"), py::arg("chosen"), py::arg("weights"),
         py::arg("groups"), py::arg("keep_groups"), py::arg("group_top"), py::arg("scale"), py::arg("weight_eps"),
         py::arg("score_kind") = 0, py::arg("normalize") = true, py::arg("bias") = py::none());

@@ -747,6 +747,23 @@ bool weight_tensor_map(const void* base, int64_t rows, int64_t cols, int box_row
   return matrix_map(base, rows, cols, box_rows, out);
 }
 
+bool strided_tensor_map(const void* base, int rank, const int64_t* dims, const int64_t* strides, const int* box,
+                        CUtensorMap* out) {
+  EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr || rank < 2 || rank > 3) return false;
+  cuuint64_t d[3], st[2];
+  cuuint32_t b[3];
+  const cuuint32_t elem[3] = {1, 1, 1};
+  for (int i = 0; i < rank; ++i) {
+    d[i] = (cuuint64_t)dims[i];
+    b[i] = (cuuint32_t)box[i];
+    if (i > 0) st[i - 1] = (cuuint64_t)strides[i - 1] * 2;
+  }
+  return fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base), d, st, b, elem,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 bool small_m_gemm_supported(int64_t tokens, int64_t features, int64_t k) {
   return tokens >= 1 && tokens <= 64 && k >= 64 && k % 8 == 0 && features >= 1 && encode_fn() != nullptr &&
          (features + kTileM - 1) / kTileM <= 0x7fffffffLL;

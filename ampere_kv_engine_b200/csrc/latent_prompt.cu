@@ -1,0 +1,438 @@
+// Prompt attention through latents, with keys and values of every head written out (bfloat16, tcgen05).
+//
+// A cache that keeps one latent per token (rank + rot_dim wide, shared by all heads) can be attended to in two ways.  In
+// the latent space a (query, key) pair costs 2 (2 rank + rot_dim) multiply-adds a head (1,088 x 2 at 512 + 64); with the
+// heads' own keys and values, made from the latents by one product, 2 (dim + rot_dim + v_dim) (320 x 2 at 128 + 64,
+// 128), plus 2 rank (dim + v_dim) per key and head once, which a portion of n queries shares.  A portion of more than a
+// few dozen tokens is far better off with the second:
+//   latent_gather           the rows of every sequence's cache that its portion can see, one under the other (each
+//                           sequence's run padded with zeros to a multiple of 128 rows, so that no key block holds rows
+//                           of two sequences)
+//   (a library product)     those rows' latents times [W_uk | W_uv] of every head: kv [rows, heads, dim + v_dim]
+//   latent_prompt_attention one CTA per (128 query tokens, head) walks the keys 128 at a time:
+//       S  = Q K^T     tcgen05.mma, M = 128, N = 128, K = dim (two 64-dim chunks) + rot_dim (one chunk: the rotated
+//                      parts, of which the key's is the gathered row's own), S in TMEM, double-buffered
+//       P  = softmax   256 threads, two per query row (64 keys each), float32, running maximum raised only by more than
+//                      2^8, P written over the scores as bfloat16 pairs
+//       O += P V       tcgen05.mma, A from TMEM, V an MN-major operand, O in TMEM
+// Warps 0-7 softmax, warp 8 copies (boxes of 128 rows by 64 dims: three for K, two for V), warp 9 issues the scores,
+// warp 10 P V.  A block's 20 MMAs of 64 tensor cycles are issued by two threads; the softmax of a block (16,384
+// exponentials, 1,024 cycles of the SM's special-function units) runs beside them.
+//
+// Measured as whole prompt steps of four latent (or two capped and two latent) layers, attention in the latent space
+// before: 2,048 tokens, 32 heads of 128 + 64, rank 512: behind a window of 1,024 7.35 -> 3.44 ms, over all keys 5.39 ->
+// 2.75 ms, after 2,048 earlier tokens 10.11 -> 2.93 ms.
+//
+// Every wait is bounded; a wait that runs out sets kWaitTimeout and the CTA frees its TMEM and leaves.
+#include "common.cuh"
+#include "launchers.h"
+#include "tcgen05.cuh"
+#include "tensor_map.h"
+
+#include <math_constants.h>
+
+namespace akv {
+
+namespace {
+
+constexpr int kRows = 128, kKeys = 128, kStages = 2;
+constexpr int kChunk = 128 * 128;                      // 128 rows of 64 dims
+constexpr int kQBytes = 3 * kChunk, kKBytes = 3 * kChunk, kVBytes = 2 * kChunk;
+constexpr int kStageBytes = kKBytes + kVBytes;
+constexpr int kSoftmax = 256, kThreads = kSoftmax + 96;
+constexpr float kLog2e = 1.4426950408889634f;
+constexpr float kRescaleThreshold = 8.f;               // log2 units
+
+struct Shared {
+  uint64_t q_full, k_full[kStages], v_full[kStages], k_empty[kStages], v_empty[kStages];
+  uint64_t s_ready[2];       // scores of a block are in TMEM buffer (block & 1)
+  uint64_t p_ready[2];       // P of a block is in tensor memory: 256 arrivals
+  uint64_t pv_done[2];       // O holds the sum through block j: barrier (j & 1), phase (j >> 1)
+  uint32_t tmem;
+  float exchange[2][2][kRows];      // [block parity][half][row]: maxima, at the end sums
+};
+constexpr int kSmemBytes = 1024 + kQBytes + kStages * kStageBytes + (int)sizeof(Shared);
+
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+      ::"r"(tc::smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(tc::smem_u32(bar))
+      : "memory");
+}
+// MN-major operand (V: one row of 128 bytes = 64 dims of one key): kChunk between the 64-dim halves (leading offset),
+// 1024 bytes between groups of 8 keys (stride offset).
+__device__ __forceinline__ uint64_t desc_mn_major(uint32_t addr) {
+  return (uint64_t)((addr & 0x3FFFF) >> 4) | ((uint64_t)(kChunk >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
+         ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+// A from tensor memory (lane = row, a 32-bit column = two consecutive K elements)
+__device__ __forceinline__ void umma_a_tmem(uint32_t tmem_d, uint32_t tmem_a, uint64_t b, uint32_t id, uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+      "}\n" ::"r"(tmem_d), "r"(tmem_a), "l"(b), "r"(id), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ void tmem_load32(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_store32(uint32_t taddr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]),
+        "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]),
+        "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_store16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_wait_store() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void pair_sync(int id) { asm volatile("barrier.cta.sync %0, 64;" ::"r"(id) : "memory"); }
+
+}  // namespace
+
+// A warp per gathered row.  Row r belongs to the last sequence of the plan whose first row is not behind r and holds its
+// key first_key + (r - first row), zeros from the context's end on.
+__global__ void __launch_bounds__(256) latent_gather_kernel(LatentGatherParams p) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (r >= p.rows) return;
+  int low = 0, high = p.num_seqs;
+  while (high - low > 1) {
+    const int mid = (low + high) >> 1;
+    if (p.plan[mid * kLatentPlanSeq] <= r) low = mid;
+    else high = mid;
+  }
+  const int32_t* seq = p.plan + low * kLatentPlanSeq;
+  const int64_t key = seq[1] + (r - seq[0]);
+  const uint4* src = nullptr;
+  if (key < seq[2]) {
+    const int64_t logical = key / p.page_size;
+    const int page = logical < p.table_width ? p.block_table[(int64_t)seq[5] * p.table_width + logical] : -1;
+    if (page < 0 || page >= p.num_pages) {
+      if (lane == 0) set_status(p.status, kBadPage);
+    } else {
+      src = reinterpret_cast<const uint4*>((const __nv_bfloat16*)p.cache + ((int64_t)page * p.page_size + key % p.page_size) * p.width);
+    }
+  }
+  uint4* dst = reinterpret_cast<uint4*>((__nv_bfloat16*)p.out + r * p.width);
+  for (int c = lane; c < p.width / 8; c += 32) dst[c] = src != nullptr ? src[c] : make_uint4(0u, 0u, 0u, 0u);
+}
+
+int launch_latent_gather(const LatentGatherParams& p, cudaStream_t stream) {
+  if (p.rows == 0) return 0;
+  const int64_t blocks = (p.rows + 7) / 8;
+  if (p.num_seqs < 1 || p.width % 8 || blocks > 0x7fffffffLL || reinterpret_cast<uintptr_t>(p.cache) % 16 ||
+      reinterpret_cast<uintptr_t>(p.out) % 16)
+    return (int)cudaErrorInvalidValue;
+  return (int)launch_chain(latent_gather_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, dim3(1, 1, 1), p);
+}
+
+__global__ void __launch_bounds__(kThreads, 1)
+latent_prompt_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap q_rot_map,
+                     const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap k_rot_map,
+                     const __grid_constant__ CUtensorMap v_map, LatentPromptParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* q_smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* kv_smem = q_smem + kQBytes;
+  Shared& s = *reinterpret_cast<Shared*>(kv_smem + kStages * kStageBytes);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  constexpr int kCopyWarp = 8, kScoreWarp = 9, kPvWarp = 10;
+  constexpr uint32_t kTmemColumns = 512;      // S: columns 0-127 and 128-255, O: columns 256-383
+
+  pdl_launch_dependents();
+  // the plan lists the tiles with the most keys first; all heads of a tile before the next tile
+  const int head = blockIdx.x;
+  const int32_t* tile = p.plan + p.num_seqs * kLatentPlanSeq + blockIdx.y * 2;
+  const int32_t* seq = p.plan + tile[0] * kLatentPlanSeq;
+  const int base = seq[0], first_key = seq[1], ctx = seq[2], n = seq[3], q0 = seq[4] + tile[1];
+  const int nq = min(kRows, n - tile[1]);
+  const int tile_pos = ctx - n + tile[1];
+  const int lo = p.window > 0 ? max(first_key, tile_pos - p.window + 1) : first_key;
+  const int lo_row = (lo - first_key) / kKeys * kKeys;
+  const int hi = tile_pos + nq;
+  const int key_begin = first_key + lo_row;
+  const int num_blocks = (hi - key_begin + kKeys - 1) / kKeys;
+
+  if (tid == 0) {
+    tc::mbar_init(&s.q_full, 1);
+    for (int i = 0; i < kStages; ++i) {
+      tc::mbar_init(&s.k_full[i], 1);
+      tc::mbar_init(&s.v_full[i], 1);
+      tc::mbar_init(&s.k_empty[i], 1);
+      tc::mbar_init(&s.v_empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(&s.s_ready[i], 1);
+      tc::mbar_init(&s.p_ready[i], kSoftmax);
+      tc::mbar_init(&s.pv_done[i], 1);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == kScoreWarp) tc::tmem_alloc(&s.tmem, kTmemColumns);
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  const uint32_t tmem = s.tmem;
+  pdl_wait();
+  bool ok = true;
+
+  if (warp == kCopyWarp) {
+    if (lane == 0) {
+      tc::mbar_expect_tx(&s.q_full, kQBytes);
+      tma_load_3d(q_smem, &q_map, 0, head, q0, &s.q_full);
+      tma_load_3d(q_smem + kChunk, &q_map, 64, head, q0, &s.q_full);
+      tma_load_3d(q_smem + 2 * kChunk, &q_rot_map, p.rank, head, q0, &s.q_full);
+      auto fetch_keys = [&](int b) -> bool {
+        const int st = b % kStages, row = base + lo_row + b * kKeys;
+        if (b >= kStages && !tc::mbar_wait(&s.k_empty[st], ((b / kStages) - 1) & 1)) return false;
+        uint8_t* dst = kv_smem + st * kStageBytes;
+        tc::mbar_expect_tx(&s.k_full[st], kKBytes);
+        tma_load_3d(dst, &k_map, 0, head, row, &s.k_full[st]);
+        tma_load_3d(dst + kChunk, &k_map, 64, head, row, &s.k_full[st]);
+        tc::tma_load_2d(dst + 2 * kChunk, &k_rot_map, p.rank, row, &s.k_full[st]);
+        return true;
+      };
+      auto fetch_values = [&](int b) -> bool {
+        const int st = b % kStages, row = base + lo_row + b * kKeys;
+        if (b >= kStages && !tc::mbar_wait(&s.v_empty[st], ((b / kStages) - 1) & 1)) return false;
+        uint8_t* dst = kv_smem + st * kStageBytes + kKBytes;
+        tc::mbar_expect_tx(&s.v_full[st], kVBytes);
+        tma_load_3d(dst, &v_map, 0, head, row, &s.v_full[st]);
+        tma_load_3d(dst + kChunk, &v_map, 64, head, row, &s.v_full[st]);
+        return true;
+      };
+      // K of a stage is free as soon as its scores are computed, V only after P V: K runs one block ahead
+      ok = fetch_keys(0);
+      for (int b = 0; b < num_blocks && ok; ++b) {
+        if (b + 1 < num_blocks) ok = fetch_keys(b + 1);
+        if (ok) ok = fetch_values(b);
+      }
+    }
+  } else if (warp == kScoreWarp) {
+    if (lane == 0) {
+      constexpr uint32_t id_s = tc::umma_idesc(kKeys);
+      const uint32_t q_addr = tc::smem_u32(q_smem);
+      if (!tc::mbar_wait(&s.q_full, 0)) ok = false;
+      for (int b = 0; b < num_blocks && ok; ++b) {
+        const int st = b % kStages;
+        // the scores of block b go into buffer b & 1, where P of block b - 2 lay: P V of that block must be done
+        if (b >= 2 && !tc::mbar_wait(&s.pv_done[b & 1], ((b - 2) >> 1) & 1)) { ok = false; break; }
+        if (!tc::mbar_wait(&s.k_full[st], (b / kStages) & 1)) { ok = false; break; }
+        tc::fence_after();
+        const uint32_t k_addr = tc::smem_u32(kv_smem + st * kStageBytes);
+#pragma unroll
+        for (int t = 0; t < 12; ++t) {
+          const uint32_t off = (t >> 2) * kChunk + (t & 3) * 32;          // chunk, then 32 bytes per k-step
+          tc::umma_bf16(tmem + (b & 1) * kKeys, tc::umma_desc(q_addr + off), tc::umma_desc(k_addr + off), id_s, t > 0 ? 1u : 0u);
+        }
+        tc::umma_commit(&s.s_ready[b & 1]);
+        tc::umma_commit(&s.k_empty[st]);
+      }
+    }
+  } else if (warp == kPvWarp) {
+    if (lane == 0) {
+      constexpr uint32_t id_o = tc::umma_idesc(128) | (1u << 16);         // B MN-major
+      for (int b = 0; b < num_blocks && ok; ++b) {
+        const int st = b % kStages;
+        if (!tc::mbar_wait(&s.p_ready[b & 1], (b >> 1) & 1)) { ok = false; break; }
+        if (!tc::mbar_wait(&s.v_full[st], (b / kStages) & 1)) { ok = false; break; }
+        tc::fence_after();
+        const uint32_t v_addr = tc::smem_u32(kv_smem + st * kStageBytes + kKBytes);
+        const uint32_t p_tmem = tmem + (b & 1) * kKeys;
+#pragma unroll
+        for (int t = 0; t < kKeys / 16; ++t)
+          umma_a_tmem(tmem + 256, p_tmem + t * 8, desc_mn_major(v_addr + t * 16 * 128), id_o, (b > 0 || t > 0) ? 1u : 0u);
+        tc::umma_commit(&s.pv_done[b & 1]);
+        tc::umma_commit(&s.v_empty[st]);
+      }
+    }
+  } else {
+    // softmax: two threads per query row, warps w and w + 4 share the TMEM lanes 32 (w % 4) .. + 31
+    const int half = warp >> 2, row = (warp & 3) * 32 + lane, pair_bar = 1 + (warp & 3);
+    const bool live = row < nq;
+    const int pos = tile_pos + row;
+    const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    const float scale_log2 = p.scale * kLog2e;
+    float m_ref = -CUDART_INF_F, l = 0.f;              // l: this half's share of the row sum
+    if (p.sink != nullptr && live) {
+      // the walk starts as if a key of that score and of value zero had come first; one half counts it
+      m_ref = p.sink[head] * kLog2e;
+      l = half == 0 ? 1.f : 0.f;
+    }
+    for (int b = 0; b < num_blocks; ++b) {
+      const int key0 = key_begin + b * kKeys + half * 64;      // this thread's first key of the block
+      if (ok && !tc::mbar_wait(&s.s_ready[b & 1], (b >> 1) & 1)) ok = false;
+      tc::fence_after();
+      uint32_t raw[2][32];
+      if (ok) {
+        tmem_load32(lane_base + (b & 1) * kKeys + half * 64, raw[0]);
+        tmem_load32(lane_base + (b & 1) * kKeys + half * 64 + 32, raw[1]);
+        tc::tmem_wait_load();
+      }
+      // most blocks lie wholly below the diagonal and inside the window: no masks there
+      const bool plain = ok && key0 + 63 <= tile_pos && (p.window <= 0 || key0 > tile_pos + nq - 1 - p.window);
+      float mx[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+      if (plain && live) {
+#pragma unroll
+        for (int j = 0; j < 64; ++j) mx[j & 3] = fmaxf(mx[j & 3], __uint_as_float(raw[j >> 5][j & 31]));
+      } else {
+#pragma unroll
+        for (int j = 0; j < 64; ++j) {
+          const int key = key0 + j;
+          const bool visible = ok && live && key <= pos && (p.window <= 0 || key > pos - p.window);
+          if (!visible) raw[j >> 5][j & 31] = 0xff800000u;     // -inf
+          mx[j & 3] = fmaxf(mx[j & 3], __uint_as_float(raw[j >> 5][j & 31]));
+        }
+      }
+      // the row's maximum over the block: this half's and the partner's.  Both have their scores in registers once they
+      // meet, so either may then write P over the other's score columns.
+      const float hmax = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale_log2;     // the scale is positive
+      s.exchange[b & 1][half][row] = hmax;
+      pair_sync(pair_bar);
+      const float bmax = fmaxf(hmax, s.exchange[b & 1][half ^ 1][row]);
+      // the reference maximum is raised only when it pays; then O and l are rescaled (each half 64 of O's columns)
+      const bool raise = bmax > m_ref + kRescaleThreshold || (m_ref == -CUDART_INF_F && bmax > -CUDART_INF_F);
+      if (__any_sync(0xffffffffu, raise)) {
+        const float alpha = (raise && m_ref != -CUDART_INF_F) ? ex2(m_ref - bmax) : 1.f;
+        if (b > 0) {
+          if (ok && !tc::mbar_wait(&s.pv_done[(b - 1) & 1], ((b - 1) >> 1) & 1)) ok = false;
+          tc::fence_after();
+          if (ok) {
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {      // 16 columns at a time: the block's scores are alive beside them
+              uint32_t o[16];
+              tc::tmem_load16(lane_base + 256 + half * 64 + c * 16, o);
+              tc::tmem_wait_load();
+#pragma unroll
+              for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+              tmem_store16(lane_base + 256 + half * 64 + c * 16, o);
+            }
+            tmem_wait_store();
+          }
+        }
+        if (raise) {
+          l *= alpha;
+          m_ref = bmax;
+        }
+      }
+      // a row that has seen no key yet subtracts 0, so that 2^(-inf - 0) = 0 and not 2^(-inf + inf)
+      const float m_sub = m_ref == -CUDART_INF_F ? 0.f : m_ref;
+      uint32_t packed[32];
+      float part[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < 64; j += 2) {
+        const float pa = ex2(fmaf(__uint_as_float(raw[j >> 5][j & 31]), scale_log2, -m_sub));
+        const float pb = ex2(fmaf(__uint_as_float(raw[(j + 1) >> 5][(j + 1) & 31]), scale_log2, -m_sub));
+        part[(j >> 1) & 3] += pa + pb;
+        __nv_bfloat162 h = __floats2bfloat162_rn(pa, pb);
+        packed[j >> 1] = *reinterpret_cast<uint32_t*>(&h);
+      }
+      if (ok) {
+        tmem_store32(lane_base + (b & 1) * kKeys + half * 32, packed);
+        tmem_wait_store();
+      }
+      l += (part[0] + part[1]) + (part[2] + part[3]);
+      tc::fence_before();
+      tc::mbar_arrive(&s.p_ready[b & 1]);
+    }
+    float (&sums)[2][kRows] = s.exchange[num_blocks & 1];
+    sums[half][row] = l;
+    pair_sync(pair_bar);
+    l = sums[0][row] + sums[1][row];
+    // the products run in order, so the last one done means all are
+    if (num_blocks > 0 && ok && !tc::mbar_wait(&s.pv_done[(num_blocks - 1) & 1], ((num_blocks - 1) >> 1) & 1)) ok = false;
+    tc::fence_after();
+    float inv = (ok && l > 0.f) ? 1.f / l : 0.f;
+    if (p.gate != nullptr && live) inv *= p.gate[(int64_t)(q0 + row) * p.heads + head];
+    __nv_bfloat16* out = (__nv_bfloat16*)p.out + ((int64_t)(q0 + row) * p.heads + head) * p.v_dim + half * 64;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      uint32_t o[32];
+      if (ok) {
+        tmem_load32(lane_base + 256 + half * 64 + c * 32, o);
+        tc::tmem_wait_load();
+      }
+      if (ok && live) {
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          if (half * 64 + c * 32 + v * 8 >= p.v_dim) break;
+          uint32_t pair[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(o[v * 8 + 2 * e]) * inv,
+                                                      __uint_as_float(o[v * 8 + 2 * e + 1]) * inv);
+            pair[e] = *reinterpret_cast<uint32_t*>(&h);
+          }
+          *reinterpret_cast<uint4*>(out + c * 32 + v * 8) = make_uint4(pair[0], pair[1], pair[2], pair[3]);
+        }
+      }
+    }
+  }
+  if (!ok && lane == 0) set_status(p.status, kWaitTimeout);
+  tc::fence_before();
+  __syncthreads();
+  if (warp == kScoreWarp) tc::tmem_free(tmem, kTmemColumns);
+}
+
+// Widths are whole 16-byte pieces (what TMA strides and the row copies need); a key head fits two 64-dim chunks, its
+// rotated part one, a value head two.
+bool latent_prompt_supported(int dim, int rot_dim, int v_dim, int rank) {
+  return dim >= 8 && dim <= 128 && dim % 8 == 0 && rot_dim >= 8 && rot_dim <= 64 && rot_dim % 8 == 0 && v_dim >= 8 &&
+         v_dim <= 128 && v_dim % 8 == 0 && rank >= 8 && rank % 8 == 0;
+}
+
+int launch_latent_prompt(const LatentPromptParams& p, cudaStream_t stream) {
+  if (p.num_tiles == 0) return 0;
+  if (!latent_prompt_supported(p.dim, p.rot_dim, p.v_dim, p.rank) || !(p.scale > 0.f) || p.heads < 1 || p.num_tiles > 65535 ||
+      p.q_stride % 8 || p.num_seqs < 1)
+    return (int)cudaErrorInvalidValue;
+  const int row = p.rank + p.rot_dim, kv = p.dim + p.v_dim;
+  CUtensorMap q_map, q_rot_map, k_map, k_rot_map, v_map;
+  const int64_t q_dims[3] = {p.dim, p.heads, p.num_tokens}, q_strides[2] = {p.dim + p.rot_dim, p.q_stride};
+  const int64_t r_dims[3] = {row, p.heads, p.num_tokens}, r_strides[2] = {row, (int64_t)p.heads * row};
+  const int64_t k_dims[3] = {p.dim, p.heads, p.rows}, kv_strides[2] = {kv, (int64_t)p.heads * kv};
+  const int64_t v_dims[3] = {p.v_dim, p.heads, p.rows};
+  const int64_t l_dims[2] = {row, p.rows}, l_strides[1] = {row};
+  const int box3[3] = {64, 1, 128}, box2[2] = {64, 128};
+  if (!strided_tensor_map(p.q, 3, q_dims, q_strides, box3, &q_map) ||
+      !strided_tensor_map(p.q_rows, 3, r_dims, r_strides, box3, &q_rot_map) ||
+      !strided_tensor_map(p.kv, 3, k_dims, kv_strides, box3, &k_map) ||
+      !strided_tensor_map((const __nv_bfloat16*)p.kv + p.dim, 3, v_dims, kv_strides, box3, &v_map) ||
+      !strided_tensor_map(p.latents, 2, l_dims, l_strides, box2, &k_rot_map))
+    return (int)cudaErrorInvalidValue;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t err = cudaFuncSetAttribute(latent_prompt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    if (err != cudaSuccess) return (int)err;
+    configured = true;
+  }
+  return (int)launch_chain(latent_prompt_kernel, dim3((unsigned)p.heads, (unsigned)p.num_tiles), dim3(kThreads), kSmemBytes,
+                           stream, dim3(1, 1, 1), q_map, q_rot_map, k_map, k_rot_map, v_map, p);
+}
+
+}  // namespace akv

@@ -255,6 +255,38 @@ int launch_scored_attention_mma(const ScoredAttentionParams& p, cudaStream_t str
 bool attention_tcgen05_scored_supported(const ScoredAttentionParams& p);
 int launch_attention_tcgen05_scored(const ScoredAttentionParams& p, cudaStream_t stream);
 
+// Prompt attention through latents with every head's keys and values written out (latent_prompt.cu).  `plan` (int32)
+// holds kLatentPlanSeq numbers per sequence: its first gathered row (a multiple of 128), the key in that row, the length
+// of its context, its new tokens, the batch row of the first of them, its row of the block table; and behind them two per
+// tile of 128 query tokens: its sequence in the plan, its first token among the sequence's new ones.
+constexpr int kLatentPlanSeq = 6;
+struct LatentGatherParams {
+  const void* cache;           // [num_pages, 1, page_size, width]
+  const int32_t* block_table;  // [sequences, table_width]
+  const int32_t* plan;
+  void* out;                   // [rows, width]
+  int64_t rows, num_pages;
+  int num_seqs, page_size, table_width, width;
+  int* status;
+};
+int launch_latent_gather(const LatentGatherParams& p, cudaStream_t stream);
+struct LatentPromptParams {
+  const void* q;               // head h of token t at t * q_stride + h * (dim + rot_dim): its unturned dims
+  const void* q_rows;          // [N, heads, rank + rot_dim]: the turned dims behind the first rank columns
+  const void* kv;              // [rows, heads, dim + v_dim]
+  const void* latents;         // [rows, rank + rot_dim]: the turned key part behind the first rank columns
+  void* out;                   // [N, heads, v_dim]
+  const int32_t* plan;
+  const float* gate;           // [N, heads] or null
+  const float* sink;           // [heads] or null
+  int64_t num_tokens, rows, q_stride;
+  int num_seqs, num_tiles, heads, dim, rot_dim, v_dim, rank, window;
+  float scale;
+  int* status;
+};
+bool latent_prompt_supported(int dim, int rot_dim, int v_dim, int rank);
+int launch_latent_prompt(const LatentPromptParams& p, cudaStream_t stream);
+
 // What stands between one product that holds [q heads | k heads | v heads | a gate column per q head] of every token
 // and the attention over them (mixer_prep.cu): q and k heads scaled to unit RMS, v blended with another layer's
 // values of the same token, k and v written to their cache slots, gates through a sigmoid.

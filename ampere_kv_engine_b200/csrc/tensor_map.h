@@ -11,4 +11,9 @@ namespace akv {
 // or refuses the shape.
 bool weight_tensor_map(const void* base, int64_t rows, int64_t cols, int box_rows, CUtensorMap* out);
 
+// Map over a bfloat16 tensor of two or three dimensions, the innermost contiguous: `dims` and `box` innermost first,
+// `strides` the elements between neighbours in the dimensions behind it; 128-byte swizzle, zeros outside.  Not cached.
+bool strided_tensor_map(const void* base, int rank, const int64_t* dims, const int64_t* strides, const int* box,
+                        CUtensorMap* out);
+
 }  // namespace akv

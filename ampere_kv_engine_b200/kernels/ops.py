@@ -496,6 +496,72 @@ def rotate_pairs(x, out, positions, inv_freq, *, heads, cols, rotary_dims, in_of
     _launched()
 
 
+LATENT_TILE = 128          # query tokens of a tile, keys of a block: a sequence's gathered rows are a multiple of it
+#: most bytes of keys and values that a step writes out; a step over longer contexts stays in the latent space
+LATENT_PLAN_BYTES = 1 << 30
+
+
+class LatentPlan:
+    """Which keys of which sequences a step's prompt portions see (``csrc/launchers.h`` describes ``numbers``)."""
+
+    def __init__(self, numbers: list[int], num_seqs: int, num_tiles: int, rows: int, tokens: int, pairs: int):
+        self.numbers, self.num_seqs, self.num_tiles, self.rows = numbers, num_seqs, num_tiles, rows
+        self.tokens, self.pairs = tokens, pairs      # new tokens; (new token, key its sequence can see) pairs
+        self.plan = None
+
+    def to(self, device):
+        staged = torch.tensor(self.numbers, dtype=torch.int32).pin_memory()
+        self.plan = staged.to(device, non_blocking=True)
+        return self
+
+
+def latent_plan(q_lens: list[int], ctx_lens: list[int], window: int) -> LatentPlan | None:
+    """The plan of the sequences with more than one new token (None without any): host lengths in, tiles with the most
+    keys first."""
+    numbers, tiles, rows, row0, tokens, pairs = [], [], 0, 0, 0, 0
+    for s, (n, c) in enumerate(zip(q_lens, ctx_lens)):
+        if n > 1:
+            first = max(0, c - n - window + 1) if window else 0
+            index = len(numbers) // 6
+            numbers += [rows, first, c, n, row0, s]
+            rows += (c - first + LATENT_TILE - 1) // LATENT_TILE * LATENT_TILE
+            tokens += n
+            pairs += n * (c - first)
+            for t in range(0, n, LATENT_TILE):
+                last = c - n + min(n, t + LATENT_TILE)
+                tiles.append((last - max(first, c - n + t - window + 1 if window else 0), index, t))
+        row0 += n
+    if not tiles:
+        return None
+    tiles.sort(key=lambda tile: -tile[0])
+    count = len(numbers) // 6
+    for _, index, t in tiles:
+        numbers += [index, t]
+    return LatentPlan(numbers, count, len(tiles), rows, tokens, pairs)
+
+
+def latent_prompt_takes(dtype: torch.dtype, device, dim: int, rot_dim: int, v_dim: int, rank: int) -> bool:
+    """Whether :func:`latent_prompt_attention` has a kernel for these widths."""
+    return dtype == torch.bfloat16 and torch.device(device).type == "cuda" and \
+        all(8 <= w <= most and w % 8 == 0 for w, most in ((dim, 128), (rot_dim, 64), (v_dim, 128), (rank, 512)))
+
+
+def latent_prompt_attention(q, q_rows, cache, block_table, plan: LatentPlan, w_kv, out, *, heads, dim, rot_dim, v_dim,
+                            rank, scale, window=0, gate=None, sink=None, status=None):
+    """Causal attention of the plan's prompt portions over latents, with every head's keys and values written out: the
+    cache rows the portions see are gathered, ``w_kv`` [heads * (dim + v_dim), rank] makes keys and values of them, and
+    each query tile walks those of its head.  ``q`` [tokens, heads * (dim + rot_dim) and more]: the unturned dims of each
+    head; ``q_rows`` [tokens, heads * (rank + rot_dim)]: the turned ones behind the first ``rank`` columns.  Writes the
+    portions' rows of ``out`` [tokens, heads * v_dim]; ``gate`` and ``sink`` as for :func:`scored_attention`."""
+    latents = torch.empty((plan.rows, rank + rot_dim), dtype=cache.dtype, device=cache.device)
+    ext().latent_gather(cache, block_table, plan.plan, latents, plan.num_seqs, status)
+    kv = torch.nn.functional.linear(latents[:, :rank], w_kv)
+    ext().latent_prompt_attention(q, q_rows, kv, latents, out, plan.plan, plan.num_seqs, plan.num_tiles, heads, dim, rot_dim,
+                                  v_dim, rank, int(window or 0), float(scale), gate, sink, status)
+    _launched(2)
+    return out
+
+
 ACTIVATIONS = {"relu2": 0, "gelu_tanh": 1, "silu": 2, "gelu": 3}
 
 

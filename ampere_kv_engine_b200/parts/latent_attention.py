@@ -13,11 +13,13 @@ What of it a mixer has is up to its parameters: without ``q_rank`` the queries c
 and the rows of an earlier schedule position (the model's schedule names it) are read, with this mixer's own queries,
 ``W_uk``, ``W_uv`` and window; the rotation may come with rescaled frequencies and a factor (``position_encoding``).
 
-Only ``c`` and ``r`` are kept per token, side by side in one cache row ``[kv_rank + rot_dim]``.  Keys and values
-are never expanded: since ``q_unrot . (W_uk c) = (W_uk^T q_unrot) . c``, the query is carried into the latent space
-(one batched product per step) and attention runs over the rows as they are stored, every head reading the same
+Only ``c`` and ``r`` are kept per token, side by side in one cache row ``[kv_rank + rot_dim]``.  Single tokens never see
+keys and values written out: since ``q_unrot . (W_uk c) = (W_uk^T q_unrot) . c``, the query is carried into the latent
+space (one batched product per step) and attention runs over the rows as they are stored, every head reading the same
 row as its key and the row's first ``kv_rank`` elements as its value; the result per head is a mix of latents (times
-the head's gate), which ``W_uv`` turns into the head's output (one more batched product).  Between the first product
+the head's gate), which ``W_uv`` turns into the head's output (one more batched product).  Prompt portions in bfloat16
+(:meth:`LatentAttention.prompt_plan`) share their keys among enough queries to have them written out for the step: one
+product makes every head's keys and values of the rows they see, and attention runs over those (``ops.latent_prompt_attention``).  Between the first product
 and the attention stands one row-wise kernel (``ops.latent_prep``; with a query latent also ``ops.rotate_pairs`` behind
 the second product).
 """
@@ -33,6 +35,13 @@ from .scored_attention import run_attention
 #: the first product's columns are padded to a multiple of this many: its rows then start on 16-byte boundaries in
 #: either precision, which the batched product that reads the queries out of them likes
 ROW_MULTIPLE = 8
+
+
+#: New tokens a portion must have, weighted by the keys it sees, for keys and values to be written out.  Measured as
+#: whole steps of four layers (us, written out against in the latent space; 32 heads of 128 + 64, rank 512, two of the
+#: layers over all keys): 16 tokens after none 827 / 870, after 2,048 913 / 994; 64 tokens 865 / 917, 965 / 1,091; 512
+#: tokens 1,112 / 1,355, 1,205 / 2,732.  At 8 tokens the two are within what such steps differ by.
+LATENT_PORTION = 16
 
 
 @register_mixer("latent_attention")
@@ -145,6 +154,27 @@ class LatentAttention(Mixer):
         self.w_uk = tensors[n["uk"]].view(H, self.head_dim, self.kv_rank).contiguous()
         self.w_uv = tensors[n["uv"]].view(H, self.v_dim, self.kv_rank).transpose(1, 2).contiguous()
         self.w_o = tensors[n["out"]].contiguous()
+        self.w_kv = None
+        if ops.latent_prompt_takes(self.dtype, self.device, self.head_dim, self.rot_dim, self.v_dim, self.kv_rank) \
+                and self.scale > 0 and (self.q_width if self.q_rank else self.w_in.shape[0]) % 8 == 0:
+            # per head its key rows and its value rows: one product writes both out for a prompt
+            self.w_kv = torch.cat((self.w_uk, tensors[n["uv"]].view(H, self.v_dim, self.kv_rank)), dim=1).flatten(0, 1)
+
+    def prompt_plan(self, ctx):
+        """The step's ``ops.LatentPlan`` if its prompt portions are better off with keys and values written out, else
+        None.  A key costs a portion 2 rank (dim + v_dim) operations a head once, and each (query, key) pair then 2 (dim
+        + rot_dim + v_dim) instead of 2 (2 rank + rot_dim), on a faster kernel."""
+        if self.w_kv is None or not any(n > 1 for n in ctx.q_lens_host):
+            return None
+        key = ("latent_prompt", self.window)
+        if key not in ctx.shared:
+            plan = ops.latent_plan(ctx.q_lens_host, ctx.ctx_lens_host, self.window)
+            worth = plan is not None and plan.pairs >= LATENT_PORTION * plan.rows
+            ctx.shared[key] = plan.to(self.device) if worth else None
+        plan = ctx.shared[key]
+        if plan is None or plan.rows * self.num_heads * (self.head_dim + self.v_dim) * 2 > ops.LATENT_PLAN_BYTES:
+            return None
+        return plan
 
     def forward(self, x, ctx, cache, residual=None):
         if cache.writes != self.own_kv:
@@ -168,15 +198,25 @@ class LatentAttention(Mixer):
                                  in_offset=D, out_offset=rank, factor=self.rotary_factor)
         else:
             q = x[:, :self.q_width]
-        # the unrotated part of every head's query, carried into the latent space: [H, tokens, D] x [H, D, rank]
-        torch.bmm(q.unflatten(1, (H, D + R))[:, :, :D].transpose(0, 1), self.w_uk,
-                  out=q_row.view(tokens, H, self.row)[:, :, :rank].transpose(0, 1))
-        mixed = torch.empty((tokens, H * rank), dtype=q.dtype, device=q.device)
-        run_attention(ctx, group, q_row, rows, rows, mixed, num_heads=H, num_kv_heads=1, v_dim=rank, scale=self.scale,
-                      window=self.window, gate=gate, sink=self.sink)
+        plan = self.prompt_plan(ctx)
         out = torch.empty((tokens, H * self.v_dim), dtype=q.dtype, device=q.device)
-        torch.bmm(mixed.view(tokens, H, rank).transpose(0, 1), self.w_uv,
-                  out=out.view(tokens, H, self.v_dim).transpose(0, 1))              # [H, tokens, v_dim]
+        single = getattr(ctx, "num_decode_tiles", 0)
+        if plan is None or single:
+            # in the latent space; where the prompt portions go the other way only the single tokens' rows matter, and
+            # where those come first only they are computed
+            count = single if plan is not None and all(n == 1 for n in ctx.q_lens_host[:single]) else tokens
+            # the unrotated part of every head's query, carried into the latent space: [H, count, D] x [H, D, rank]
+            torch.bmm(q[:count].unflatten(1, (H, D + R))[:, :, :D].transpose(0, 1), self.w_uk,
+                      out=q_row.view(tokens, H, self.row)[:count, :, :rank].transpose(0, 1))
+            mixed = torch.empty((tokens, H * rank), dtype=q.dtype, device=q.device)
+            run_attention(ctx, group, q_row, rows, rows, mixed, num_heads=H, num_kv_heads=1, v_dim=rank, scale=self.scale,
+                          window=self.window, gate=gate, sink=self.sink, single_only=plan is not None)
+            torch.bmm(mixed.view(tokens, H, rank)[:count].transpose(0, 1), self.w_uv,
+                      out=out.view(tokens, H, self.v_dim)[:count].transpose(0, 1))              # [H, count, v_dim]
+        if plan is not None:
+            ops.latent_prompt_attention(q, q_row, rows, group.block_table, plan, self.w_kv, out, heads=H, dim=D, rot_dim=R,
+                                        v_dim=self.v_dim, rank=rank, scale=self.scale, window=self.window, gate=gate,
+                                        sink=self.sink, status=ctx.status)
         if residual is not None:
             summed = ops.linear_into_residual(out, self.w_o, residual, status=ctx.status)
             if summed is not None:

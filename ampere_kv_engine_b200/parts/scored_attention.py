@@ -162,8 +162,8 @@ class ScoredAttention(Mixer):
 
 def run_attention(ctx, group, q, k_cache, v_cache, out, *, num_heads, num_kv_heads, v_dim, scale, window=0, chunk=0,
                   softcap=0.0, slopes=None, gate=None, plain=False, keep_first=0, sigmoid_weights=False, head_bias=None,
-                  out_scale=1.0, sink=None) -> None:
-    """``ops.scored_attention`` over the step's tiles: the single-token tiles of a mixed step (they come first) apart
+                  out_scale=1.0, sink=None, single_only=False) -> None:
+    """``ops.scored_attention`` over the step's tiles (``single_only``: the single-token ones of a mixed step alone): the single-token tiles of a mixed step (they come first) apart
     from the prompt tiles, each with the number of key splits that fills the GPU.  ``plain``: nothing is done to the
     scores and the plain kernels take the sizes: ``ops.paged_attention`` runs instead."""
     group_size = num_heads // num_kv_heads
@@ -171,7 +171,7 @@ def run_attention(ctx, group, q, k_cache, v_cache, out, *, num_heads, num_kv_hea
                                                           k_cache.shape[2])
     first = getattr(ctx, "num_decode_tiles", 0)
     for lo, hi, q_tile in ((0, first, 1), (first, ctx.num_tiles, ctx.q_tile)):
-        if hi <= lo:
+        if hi <= lo or (single_only and lo == first):
             continue
         longest, mean = ctx.decode_contexts if q_tile == 1 else (ctx.max_context, ctx.max_context)
         for limit in (window + keep_first if window else 0, chunk):
