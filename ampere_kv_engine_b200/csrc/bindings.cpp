@@ -1488,6 +1488,7 @@ void linear_scan(const Tensor& x, Tensor& state, const Tensor& cu_q, const Tenso
   p.state = state.data_ptr<float>();
   p.state_stride = state.stride(0);
   p.cu_q = cu_q.data_ptr<int>();
+  p.num_slots = (int)state.size(0);
   p.state_slots = state_slots.data_ptr<int>();
   p.out = out.data_ptr<float>();
   p.num_tokens = n;

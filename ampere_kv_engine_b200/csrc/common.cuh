@@ -87,6 +87,31 @@ __device__ __forceinline__ float activation_value(float z, int kind) {
   return z / (1.f + expf(-z));
 }
 
+// Two float32 operations in one instruction (packed in a register pair, each rounded as its scalar form is): for kernels
+// that are bound by instruction issue.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)),
+        "l"(reinterpret_cast<unsigned long long&>(c)));
+  return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<unsigned long long&>(d))
+      : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+  return d;
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -97,6 +122,38 @@ __device__ __forceinline__ float warp_max(float v) {
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
+
+// Sums over groups of RL neighbouring lanes (8, 16 or 32) of eight values each: afterwards lane i of a group holds the sum
+// of value spread_index<RL>(i).  Half of the values travel in each of the first three steps: 7 + log2(RL / 8) shuffles in
+// log2(RL) steps instead of 8 log2(RL).
+template <int RL>
+__device__ __forceinline__ int spread_index(int lane) {
+  return ((lane & (RL / 2)) ? 4 : 0) + ((lane & (RL / 4)) ? 2 : 0) + ((lane & (RL / 8)) ? 1 : 0);
+}
+template <int RL>
+__device__ __forceinline__ float spread_sum8(const float (&v)[8], int lane) {
+  const bool b2 = (lane & (RL / 2)) != 0, b1 = (lane & (RL / 4)) != 0, b0 = (lane & (RL / 8)) != 0;
+  float four[4], two[2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) four[i] = (b2 ? v[i + 4] : v[i]) + __shfl_xor_sync(0xffffffffu, b2 ? v[i] : v[i + 4], RL / 2);
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    two[i] = (b1 ? four[i + 2] : four[i]) + __shfl_xor_sync(0xffffffffu, b1 ? four[i] : four[i + 2], RL / 4);
+  float sum = (b0 ? two[1] : two[0]) + __shfl_xor_sync(0xffffffffu, b0 ? two[0] : two[1], RL / 8);
+#pragma unroll
+  for (int o = RL / 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  return sum;
+}
+
+// 16 or 4 bytes from global to shared memory, asynchronously.
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* smem, const void* global) {
+  const unsigned at = (unsigned)__cvta_generic_to_shared(smem);
+  if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(at), "l"(global) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(at), "l"(global) : "memory");
+}
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void copy_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // Sum over a whole block (any multiple of 32 threads up to 1024); every thread gets the result.
 // `scratch` must hold 33 floats of shared memory.
@@ -192,6 +249,20 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // Launch with the programmatic-stream-serialization attribute (and, if cluster_z/cluster_y > 1, a cluster).
 // AKV_NO_PDL=1 in the environment launches without it (for comparisons).
 bool pdl_enabled();
+
+// Launch without that attribute: for kernels of few, long-running blocks.  Blocks that start early are placed wherever the
+// previous kernel's last blocks leave room, several to an SM while others stay empty, and a kernel whose time is its longest
+// block's pays for that to its end (measured: a scan of 64 blocks over 2,048 tokens 1,000 us so, 405 us spread out).
+template <typename... KernelArgs, typename... Args>
+inline cudaError_t launch_alone(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                Args&&... args) {
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = block;
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  return cudaLaunchKernelEx(&config, kernel, static_cast<KernelArgs>(args)...);
+}
 
 template <typename... KernelArgs, typename... Args>
 inline cudaError_t launch_chain(void (*kernel)(KernelArgs...), dim3 grid, dim3 block, size_t smem,

@@ -9,15 +9,16 @@
 //                (token, head).
 //   delta_scan:  blocks per (sequence, head, slice of the value columns) walk the step's tokens of that sequence in
 //                order:  S *= decay;  u = beta (v - S^T k);  S += k u^T;  o = S^T q.
-//                A thread group of up to 8 lanes owns one value column of S (in registers for the whole step); the
+//                A thread group of up to 8 lanes owns one value column of S (in registers for the whole step; prompts
+//                mostly take a form in which a thread owns parts of four columns); the
 //                two products are a few multiply-adds per lane and a shuffle reduction over the group; tokens are
 //                staged through shared memory in chunks, so a token costs no block barrier.  A second kernel applies
 //                the output norm o / sqrt(mean(o^2) + eps) * w * silu(gate) (or sigmoid(gate)) to all tokens in parallel and, in further
 //                blocks, moves each sequence's last taps - 1 convolution inputs into the state.
 //
 // The walk is token by token whatever the step holds, so the state after a token does not depend on how the
-// tokens were cut into steps.  A sequence whose state slot is negative (padding of a captured step) is left alone
-// and its output rows are zero.
+// tokens were cut into steps, but for the order in which the lanes' parts of a sum are added.  A sequence whose state
+// slot is negative (padding of a captured step) is left alone and its output rows are zero.
 #include "common.cuh"
 #include "launchers.h"
 
@@ -38,6 +39,7 @@ __device__ __forceinline__ int sequence_of(const int32_t* cu_q, int num_seqs, in
 }
 
 constexpr int kMaxPerLane = kDeltaMaxDim / 32;
+constexpr int kWalkColumns = 32, kWalkChunk = 16;      // value columns per block, tokens per chunk of the walk in tiles
 
 __device__ __forceinline__ float load_any(const void* p, int64_t i, int dtype) {
   return dtype == kBFloat16 ? __bfloat162float(((const __nv_bfloat16*)p)[i]) : ((const float*)p)[i];
@@ -399,6 +401,223 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(DeltaParams p, int cols
   }
 }
 
+// The scan of a prompt whose heads' rows are whole 16-byte pieces.  Two things bound the form above there: the way from
+// shared memory into registers (128 bytes a cycle and SM: a thread reads 2 x EPT numbers of q and k for EPT elements of S),
+// and the chain of a token, which a warp issues in order: two sums over lanes, one after the other.  Here a thread owns
+// QUADS quads of rows x 4 columns of S in pairs (RL lanes x 4 QUADS rows cover the dim, a block again 32 columns), so that
+// 16 numbers serve 32 elements.  What a token needs of S, S^T k, and what the token before it is read out with, S^T q, are
+// taken from the same S: eight sums, which go through ONE exchange over RL lanes.  A token's numbers stand in registers one
+// token ahead; tokens arrive kWalkChunk at a time by asynchronous copies, a warp a token.  16 heads of 128 x 128 (us, before | now):
+// one sequence of 2,048 tokens 640 | 575, three of 1,501, 301 and 246 556 | 554, seven of 300 398 | 206; 32 heads 656 | 591,
+// 855 | 724, 695 | 349.
+template <int RL, int QUADS, bool CHANNEL>
+__global__ void __launch_bounds__(RL * 8) delta_walk_kernel(DeltaParams p, int ept, int lanes) {
+  constexpr int kRowsPadded = RL * 4 * QUADS, kPairs = 2 * QUADS, kChunk = kWalkChunk, kWarps = RL / 4;
+  constexpr int kVecs = CHANNEL ? 3 : 2;
+  constexpr int kToken = kVecs * kRowsPadded + kWalkColumns + 4;      // [q | k (| decays) | v | beta, decay]
+  constexpr int kPieces = (kVecs * kRowsPadded + kWalkColumns + 127) / 128;
+  extern __shared__ __align__(16) float smem[];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int s = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * kWalkColumns;
+  const int G = p.num_kv_heads, H = p.num_heads, D = p.head_dim, V = p.v_dim;
+  const int channels = 2 * G * D + H * V;
+  const int64_t first = p.cu_q[s];
+  const int n = (int)(p.cu_q[s + 1] - first);
+  const int slot = p.state_slots[s];
+  if (n <= 0 || first < 0 || first + n > p.num_tokens) return;
+  const int mine_cols = min(kWalkColumns, V - col0);
+  float* scratch = p.scratch + first * H * V + (int64_t)h * V + col0;
+  if (slot < 0 || slot >= p.num_slots) {
+    for (int i = threadIdx.x; i < n * mine_cols; i += blockDim.x) scratch[(int64_t)(i / mine_cols) * H * V + i % mine_cols] = 0.f;
+    return;
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int rl = lane % RL;
+  const int col = (warp * (32 / RL) + lane / RL) * 4;                 // the thread's first column in the block
+  const int g = h / (H / G);
+  // quad q of the thread's rows: 4 RL q + 4 rl .. + 3, and where it lies in the state slot
+  float* memory = p.state + (int64_t)slot * p.state_stride + (int64_t)h * V * lanes * ept;
+  auto place = [&](int q, int c) -> float4* {
+    const int d = q * 4 * RL + 4 * rl;
+    if (d >= lanes * ept || col + c >= mine_cols) return nullptr;
+    return reinterpret_cast<float4*>(memory + (((int64_t)(d % ept / 4) * V + col0 + col + c) * lanes + d / ept) * 4);
+  };
+  float2 S[kPairs][4];                                                 // [pair of rows][column]
+#pragma unroll
+  for (int q = 0; q < QUADS; ++q)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float4* at = place(q, c);
+      const float4 v = at != nullptr ? *at : make_float4(0.f, 0.f, 0.f, 0.f);
+      S[2 * q][c] = make_float2(v.x, v.y);
+      S[2 * q + 1][c] = make_float2(v.z, v.w);
+    }
+  // this lane's pieces of a token
+  const float* piece_src[kPieces];
+  int64_t piece_stride[kPieces];
+  int piece_dst[kPieces];
+#pragma unroll
+  for (int r = 0; r < kPieces; ++r) {
+    const int i = (lane + 32 * r) * 4;
+    const float* qkv = p.qkv + first * channels;
+    piece_src[r] = nullptr;
+    piece_stride[r] = channels;
+    piece_dst[r] = 0;
+    if (i < D) {
+      piece_src[r] = qkv + g * D + i;
+      piece_dst[r] = i;
+    } else if (i < 2 * D) {
+      piece_src[r] = qkv + G * D + g * D + (i - D);
+      piece_dst[r] = kRowsPadded + (i - D);
+    } else if (i < 2 * D + mine_cols) {
+      piece_src[r] = qkv + 2 * G * D + h * V + col0 + (i - 2 * D);
+      piece_dst[r] = kVecs * kRowsPadded + (i - 2 * D);
+    } else if (CHANNEL && i < 3 * D + mine_cols) {
+      const int d = i - 2 * D - mine_cols;
+      piece_src[r] = p.coef + first * p.coef_stride + H + h * D + d;
+      piece_dst[r] = 2 * kRowsPadded + d;
+      piece_stride[r] = p.coef_stride;
+    }
+  }
+  auto copy = [&](float* buffer, int t0, int count) {
+    for (int t = warp; t < count; t += kWarps) {
+#pragma unroll
+      for (int r = 0; r < kPieces; ++r)
+        if (piece_src[r] != nullptr)
+          copy_async<16>(buffer + t * kToken + piece_dst[r], piece_src[r] + (int64_t)(t0 + t) * piece_stride[r]);
+      if (lane < (CHANNEL ? 1 : 2))
+        copy_async<4>(buffer + t * kToken + kVecs * kRowsPadded + kWalkColumns + lane,
+                      p.coef + (first + t0 + t) * p.coef_stride + lane * H + h);
+    }
+    copy_async_commit();
+  };
+  struct Token {
+    float2 q[kPairs], k[kPairs], g[CHANNEL ? kPairs : 1];
+    float v, beta, decay;                                              // v: of the column that this lane ends a sum with
+  };
+  // a lane ends an exchange with the sum of one column: of S^T k or (reads_out) of S^T q
+  const bool reads_out = spread_index<RL>(lane) >= 4;
+  const int own = col + (spread_index<RL>(lane) & 3);
+  const bool stores = reads_out && rl % (RL / 8 > 0 ? RL / 8 : 1) == 0 && own < mine_cols;
+  auto load = [&](Token& x, const float* row) {
+#pragma unroll
+    for (int i = 0; i < QUADS; ++i) {
+      const float4 q = *reinterpret_cast<const float4*>(row + i * 4 * RL + 4 * rl);
+      const float4 k = *reinterpret_cast<const float4*>(row + kRowsPadded + i * 4 * RL + 4 * rl);
+      x.q[2 * i] = make_float2(q.x, q.y);
+      x.q[2 * i + 1] = make_float2(q.z, q.w);
+      x.k[2 * i] = make_float2(k.x, k.y);
+      x.k[2 * i + 1] = make_float2(k.z, k.w);
+      if constexpr (CHANNEL) {
+        const float4 d = *reinterpret_cast<const float4*>(row + 2 * kRowsPadded + i * 4 * RL + 4 * rl);
+        x.g[2 * i] = make_float2(d.x, d.y);
+        x.g[2 * i + 1] = make_float2(d.z, d.w);
+      }
+    }
+    x.v = row[kVecs * kRowsPadded + own];
+    x.beta = row[kVecs * kRowsPadded + kWalkColumns];
+    x.decay = CHANNEL ? 1.f : row[kVecs * kRowsPadded + kWalkColumns + 1];
+  };
+  float2 read[kPairs];                                                 // q of the token before
+#pragma unroll
+  for (int r = 0; r < kPairs; ++r) read[r] = make_float2(0.f, 0.f);
+  // Token x; `before`: where the output of the token before it goes.
+  auto step = [&](const Token& x, float* before, bool any_before) {
+    float2 sum[8];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      sum[4 + c] = mul2(S[0][c], read[0]);
+#pragma unroll
+      for (int r = 1; r < kPairs; ++r) sum[4 + c] = fma2(S[r][c], read[r], sum[4 + c]);
+    }
+    if constexpr (CHANNEL) {
+      // every row of S by its own decay first; what follows is then the form with one decay, at one
+#pragma unroll
+      for (int r = 0; r < kPairs; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) S[r][c] = mul2(S[r][c], x.g[r]);
+    }
+    float parts[8];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      sum[c] = mul2(S[0][c], x.k[0]);
+#pragma unroll
+      for (int r = 1; r < kPairs; ++r) sum[c] = fma2(S[r][c], x.k[r], sum[c]);
+      parts[c] = sum[c].x + sum[c].y;
+      parts[4 + c] = sum[4 + c].x + sum[4 + c].y;
+    }
+    const float total = spread_sum8<RL>(parts, lane);
+    if (any_before && stores) before[own] = total;
+    const float u = x.beta * (x.v - x.decay * total);                  // of column `own`, in the lanes of S^T k
+    const float2 dd = make_float2(x.decay, x.decay);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float uc = __shfl_sync(0xffffffffu, u, (lane & ~(RL - 1)) | ((c >> 1) * (RL / 4)) | ((c & 1) * (RL / 8)));
+      const float2 uu = make_float2(uc, uc);
+#pragma unroll
+      for (int r = 0; r < kPairs; ++r) S[r][c] = fma2(x.k[r], uu, CHANNEL ? S[r][c] : mul2(S[r][c], dd));
+    }
+#pragma unroll
+    for (int r = 0; r < kPairs; ++r) read[r] = x.q[r];
+  };
+  // rows beyond the dim and columns beyond the width stay zero in both buffers
+  for (int i = threadIdx.x; i < (2 * kChunk + 1) * kToken; i += blockDim.x) smem[i] = 0.f;
+  __syncthreads();
+  copy(smem, 0, min(kChunk, n));
+  copy_async_wait_all();
+  __syncthreads();
+  const int64_t wide = (int64_t)H * V;
+  for (int t0 = 0; t0 < n; t0 += kChunk) {
+    const int count = min(kChunk, n - t0), next = min(kChunk, n - t0 - kChunk);
+    const float* buffer = smem + ((t0 / kChunk) & 1) * kChunk * kToken;
+    if (next > 0) copy(smem + (((t0 / kChunk) + 1) & 1) * kChunk * kToken, t0 + kChunk, next);
+    float* to = scratch + (int64_t)t0 * wide;
+    Token even, odd;
+    load(even, buffer);
+    if (count == kChunk) {
+      // no branch between tokens, so that one's read-out can stand among the next one's instructions (the load behind the
+      // last token brings nothing that is used; there is room for it behind the second buffer)
+#pragma unroll 2
+      for (int t = 0; t < kChunk; t += 2) {
+        load(odd, buffer + (t + 1) * kToken);
+        step(even, to + (t - 1) * wide, t0 + t > 0);
+        load(even, buffer + (t + 2) * kToken);
+        step(odd, to + t * wide, true);
+      }
+    } else {
+      for (int t = 0; t < count; ++t) {
+        load(odd, buffer + (t + 1) * kToken);
+        step(even, to + (t - 1) * wide, t0 + t > 0);
+        even = odd;
+      }
+    }
+    copy_async_wait_all();
+    __syncthreads();
+  }
+  {
+    // the last token's read-out
+    float parts[8];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      float2 sum = mul2(S[0][c], read[0]);
+#pragma unroll
+      for (int r = 1; r < kPairs; ++r) sum = fma2(S[r][c], read[r], sum);
+      parts[c] = 0.f;
+      parts[4 + c] = sum.x + sum.y;
+    }
+    const float total = spread_sum8<RL>(parts, lane);
+    if (stores) scratch[(n - 1) * wide + own] = total;
+  }
+#pragma unroll
+  for (int q = 0; q < QUADS; ++q)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      float4* at = place(q, c);
+      if (at != nullptr) *at = make_float4(S[2 * q][c].x, S[2 * q][c].y, S[2 * q + 1][c].x, S[2 * q + 1][c].y);
+    }
+}
+
 // What follows the scan, in one launch.  Blocks [0, norm_blocks): the output norm and gate, a warp per (token, head):
 // o / sqrt(mean(o^2) + eps) * w * silu(gate) or sigmoid(gate), times a factor.  The blocks after them: the convolutions' memory, a thread per
 // (sequence, channel): the last taps - 1 inputs of [what was there before | this step's rows]; a thread reads all it
@@ -453,6 +672,20 @@ __global__ void __launch_bounds__(128) delta_finish_kernel(DeltaParams p, int no
     if (i < keep) before[(int64_t)i * channels + c] = kept[i];
 }
 
+template <int RL, int QUADS, bool CHANNEL>
+static int launch_walk(const DeltaParams& p, const ScanShape& shape, cudaStream_t stream) {
+  constexpr int kToken = (CHANNEL ? 3 : 2) * RL * 4 * QUADS + kWalkColumns + 4;
+  const size_t smem = (2 * (size_t)kWalkChunk + 1) * kToken * sizeof(float);
+  auto kernel = delta_walk_kernel<RL, QUADS, CHANNEL>;
+  if (smem > 48 * 1024) {
+    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err != cudaSuccess) return (int)err;
+  }
+  const int slices = (p.v_dim + kWalkColumns - 1) / kWalkColumns;
+  return (int)launch_alone(kernel, dim3((unsigned)p.num_seqs, (unsigned)p.num_heads, (unsigned)slices), dim3(RL * 8), smem,
+                           stream, p, shape.ept, shape.lanes);
+}
+
 template <int EPT, int LANES, int CHUNK, bool CHANNEL>
 static int launch_scan_chunk(const DeltaParams& p, const ScanShape& shape, cudaStream_t stream) {
   const int threads = shape.threads;
@@ -469,11 +702,19 @@ static int launch_scan_chunk(const DeltaParams& p, const ScanShape& shape, cudaS
 }
 
 // Steps of about a token per sequence (decoding) stage two tokens at a time: fewer registers and less shared memory
-// per block, so more blocks share an SM while the state streams through; prompts stage the largest chunk that fits.
+// per block, so more blocks share an SM while the state streams through.  Prompts whose heads' rows are whole 16-byte
+// pieces walk in register tiles; others stage the largest chunk that fits.
 template <int EPT, int LANES, bool CHANNEL>
 static int launch_scan_form(const DeltaParams& p, const ScanShape& shape, cudaStream_t stream) {
   constexpr int kLong = EPT >= 32 ? 8 : 16;
   if (p.num_tokens <= 2 * (int64_t)p.num_seqs) return launch_scan_chunk<EPT, LANES, 2, CHANNEL>(p, shape, stream);
+  const int channels = 2 * p.num_kv_heads * p.head_dim + p.num_heads * p.v_dim;
+  if (p.head_dim % 4 == 0 && p.v_dim % 4 == 0 && channels % 4 == 0 && reinterpret_cast<uintptr_t>(p.qkv) % 16 == 0 &&
+      (!CHANNEL || (p.num_heads % 4 == 0 && p.coef_stride % 4 == 0 && reinterpret_cast<uintptr_t>(p.coef) % 16 == 0))) {
+    if (p.head_dim <= 64) return launch_walk<8, 2, CHANNEL>(p, shape, stream);
+    if (p.head_dim <= 128) return launch_walk<16, 2, CHANNEL>(p, shape, stream);
+    return launch_walk<32, 2, CHANNEL>(p, shape, stream);
+  }
   if (shape.chunk < kLong) return (int)cudaErrorInvalidValue;
   return launch_scan_chunk<EPT, LANES, kLong, CHANNEL>(p, shape, stream);
 }

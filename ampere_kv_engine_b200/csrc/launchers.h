@@ -516,6 +516,7 @@ struct LinearScanParams {
   float* out;                  // [N, NH * DV] float32
   int64_t num_tokens;
   int num_seqs, num_heads, head_dim, v_dim, mode, dtype;
+  int num_slots;               // rows of `state`
   int qk_group;                // heads that share one q and one k (0 or 1: every head its own)
   int decay_off;               // kTokenDecay: column of x where the token's decays (a float per head) begin
   // filled in by the launcher: where the prompt form's staging warps find q, k and v in `act`

@@ -18,8 +18,9 @@
 //   Decode form (steps of a token or two per sequence): a column's threads are neighbouring lanes and add up their
 //   parts of a token's output with shuffles; every thread stages its share of the next tokens itself (loads,
 //   activations, gates).
-//   Prompt form (everything else): a kernel of its own first writes every token's q, a-or-k and v after activations
-//   and gates as float32 (once per token, not once per block of a head's value slices).  In the scan a warp holds
+//   Prompt forms (everything else): a kernel of its own first writes every token's q, a-or-k and v after activations
+//   and gates as float32 (once per token, not once per block of a head's value slices).  Where the heads' rows are whole
+//   16-byte pieces, linear_walk_kernel then walks them in register tiles; otherwise in the scan a warp holds
 //   the same rows of all 32 columns, so its reads of q and of the gates are broadcasts; it leaves its part of every
 //   token's output in shared memory, and when the chunk is walked the walking warps add the parts up, a thread per
 //   (token, column).  Further warps do nothing but copy the next chunk from the float32 scratch, asynchronously.
@@ -59,53 +60,61 @@ __host__ __device__ constexpr int scan_rounds(int rows, int producers) {
   return producers > 0 ? (2 * 8 * rows + kScanColumns + producers - 1) / producers : 3;
 }
 
-__device__ __forceinline__ void cp_async_16(void* smem, const void* global) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(global)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.commit_group;" ::: "memory");
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-}
-__device__ __forceinline__ void cp_async_4(void* smem, const void* global) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(global)
-               : "memory");
-}
-
 // act[t] = [q (NH * D) | a or k (NH * D) | v (NH * DV)] of token t after activations and gates, float32: what every
 // block of a head's value slices would otherwise work out again for itself while it stages a prompt's tokens.
-template <typename T, int MODE>
-__global__ void linear_prep_kernel(LinearScanParams p, int width) {
+// A thread takes VEC neighbouring columns (four where every boundary between the parts and every row lies on a whole
+// group of four: 2,048 tokens of 12,288 columns 34 us against 53).
+template <typename T, int VEC>
+__device__ __forceinline__ void load_columns(const T* from, float (&out)[VEC]) {
+  if constexpr (VEC == 1) {
+    out[0] = to_float<T>(*from);
+  } else if constexpr (sizeof(T) == 4) {
+    const float4 v = *reinterpret_cast<const float4*>(from);
+    out[0] = v.x; out[1] = v.y; out[2] = v.z; out[3] = v.w;
+  } else {
+    const uint2 v = *reinterpret_cast<const uint2*>(from);
+    out[0] = __uint_as_float(v.x << 16);
+    out[1] = __uint_as_float(v.x & 0xffff0000u);
+    out[2] = __uint_as_float(v.y << 16);
+    out[3] = __uint_as_float(v.y & 0xffff0000u);
+  }
+}
+
+template <typename T, int MODE, int VEC>
+__global__ void __launch_bounds__(256) linear_prep_kernel(LinearScanParams p, int width) {
   pdl_launch_dependents();
   pdl_wait();
   const int qk = p.num_heads * p.head_dim;
   const int64_t t = blockIdx.x;                        // a block row per token, blockIdx.y over its columns
   const T* row = (const T*)p.x + t * p.x_stride;
-  for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < width; c += gridDim.y * blockDim.x) {
-    float y;
-    if (c < qk) {
-      y = silu_f(to_float<T>(row[p.q_off + c]));
-    } else if (c < 2 * qk) {
-      const int ch = c - qk;
-      const float z = to_float<T>(row[p.k_off + ch]);
-      if (MODE == kGatedWrite) {
-        const float low = p.lower[ch];
-        y = low + (1.f - low) * sigmoid_f(z + (p.gate_bias != nullptr ? p.gate_bias[ch] : 0.f));
-      } else {
-        y = silu_f(z);
-      }
+  for (int c = (blockIdx.y * blockDim.x + threadIdx.x) * VEC; c < width; c += gridDim.y * blockDim.x * VEC) {
+    const int part = c < qk ? 0 : (c < 2 * qk ? 1 : 2);
+    const int ch = c - part * qk;
+    float z[VEC], y[VEC];
+    load_columns<T, VEC>(row + (part == 0 ? p.q_off : (part == 1 ? p.k_off : p.v_off)) + ch, z);
+    if (MODE == kGatedWrite && part == 1) {
+      float low[VEC], bias[VEC];
+      load_columns<float, VEC>(p.lower + ch, low);
+      if (p.gate_bias != nullptr) load_columns<float, VEC>(p.gate_bias + ch, bias);
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) y[i] = low[i] + (1.f - low[i]) * sigmoid_f(z[i] + (p.gate_bias != nullptr ? bias[i] : 0.f));
+    } else if (MODE == kGatedWrite && part == 2) {
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) y[i] = z[i];
     } else {
-      const float z = to_float<T>(row[p.v_off + c - 2 * qk]);
-      y = MODE == kGatedWrite ? z : silu_f(z);
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) y[i] = silu_f(z[i]);
     }
-    p.act[t * width + c] = y;
+    float* to = p.act + t * width + c;
+    if constexpr (VEC == 4) *reinterpret_cast<float4*>(to) = make_float4(y[0], y[1], y[2], y[3]);
+    else *to = y[0];
   }
 }
 
 // PRODUCERS == 0: the decode form.  PRODUCERS > 0: the prompt form with that many further threads that only copy
 // the next chunk from p.act into shared memory beside the walk of the current one.
 template <typename T, int MODE, int ROWS, int CHUNK, int PRODUCERS>
-__global__ void __launch_bounds__(256 + PRODUCERS)
+__global__ void __launch_bounds__(256 + PRODUCERS, 1)
 linear_scan_kernel(LinearScanParams p, int lanes, int slices) {
   constexpr int kRounds = scan_rounds(ROWS, PRODUCERS);
   constexpr bool kPrepared = MODE == kPlainDecay || MODE == kTokenDecay;     // no activation, float32 input
@@ -143,10 +152,10 @@ linear_scan_kernel(LinearScanParams p, int lanes, int slices) {
 
   float* mem = p.state + (int64_t)slot * p.state_stride +
                ((int64_t)head * slices + slice) * ROWS * (int64_t)threads + col * lanes + sub;
-  float S[ROWS];
+  float2 S[ROWS / 2];      // neighbouring rows in pairs: every operation on them is one on two
   if (walker) {
 #pragma unroll
-    for (int r = 0; r < ROWS; ++r) S[r] = mem[(int64_t)r * threads];
+    for (int r = 0; r < ROWS; r += 2) S[r / 2] = make_float2(mem[(int64_t)r * threads], mem[(int64_t)(r + 1) * threads]);
   }
   const float decay = (MODE == kConstantDecay || MODE == kPlainDecay) ? p.decay[head] : 0.f;
 
@@ -217,16 +226,13 @@ linear_scan_kernel(LinearScanParams p, int lanes, int slices) {
       }
     }
   };
-  // the same from the scratch that the preparing kernel filled (prompt form): asynchronous copies of 16 bytes where
-  // the widths allow it, of 4 otherwise, all of a chunk in flight at once
+  // the same from the scratch that the preparing kernel filled (prompt form): asynchronous copies, all of a chunk in
+  // flight at once
   auto stage_copy = [&](float* buffer, int first, int count) {
     const int64_t width = p.act_stride;
-    const bool wide_copy = D % 4 == 0 && DV % 4 == 0 && p.act_aligned;
-    const int step = wide_copy ? 4 : 1;
-    const int per = fetch_per_token / step;
     const float* base = p.act + (int64_t)(t0 + first) * width;
-    for (int e = stage_id; e < count * per; e += stagers) {
-      const int t = e / per, i = (e % per) * step;
+    for (int e = stage_id; e < count * fetch_per_token; e += stagers) {
+      const int t = e / fetch_per_token, i = e % fetch_per_token;
       const float* from = base + (int64_t)t * width;
       float* to = buffer + t * per_token;
       if (i < D) {
@@ -239,40 +245,33 @@ linear_scan_kernel(LinearScanParams p, int lanes, int slices) {
         from += p.act_v_off + head * DV + slice * kScanColumns + (i - 2 * D);
         to += 2 * vec + (i - 2 * D);
       }
-      if (wide_copy) cp_async_16(to, from);
-      else cp_async_4(to, from);
+      copy_async<4>(to, from);
     }
     if (MODE == kTokenDecay) {
       for (int t = stage_id; t < count; t += stagers)
-        cp_async_4(buffer + t * per_token + 2 * vec + kScanColumns, base + (int64_t)t * width + p.decay_off + head);
+        copy_async<4>(buffer + t * per_token + 2 * vec + kScanColumns, base + (int64_t)t * width + p.decay_off + head);
     }
-    cp_async_wait_all();
+    copy_async_commit();
+    copy_async_wait_all();
   };
   // a token's q, a and v applied to this thread's rows of S; returns its part of the token's output
   auto apply_loaded = [&](const float4 (&qs)[ROWS / 4], const float4 (&as)[ROWS / 4], float v, float decay) -> float {
-    float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
+    float2 o01 = make_float2(0.f, 0.f), o23 = o01;
+    const float2 vv = make_float2(v, v), minus = make_float2(-v, -v), dd = make_float2(decay, decay);
+    auto step = [&](float2 old, float2 a) -> float2 {
+      // f S + (1 - f) v as v + f (S - v); the others k v + decay S
+      if (MODE == kGatedWrite) return fma2(a, add2(old, minus), vv);
+      return fma2(a, vv, mul2(dd, old));
+    };
 #pragma unroll
     for (int r4 = 0; r4 < ROWS / 4; ++r4) {
       const float4 q = qs[r4], a = as[r4];
-      const int r = r4 * 4;
-      if (MODE == kGatedWrite) {
-        // f S + (1 - f) v as v + f (S - v): two operations per entry
-        S[r] = fmaf(a.x, S[r] - v, v);
-        S[r + 1] = fmaf(a.y, S[r + 1] - v, v);
-        S[r + 2] = fmaf(a.z, S[r + 2] - v, v);
-        S[r + 3] = fmaf(a.w, S[r + 3] - v, v);
-      } else {
-        S[r] = fmaf(a.x, v, decay * S[r]);
-        S[r + 1] = fmaf(a.y, v, decay * S[r + 1]);
-        S[r + 2] = fmaf(a.z, v, decay * S[r + 2]);
-        S[r + 3] = fmaf(a.w, v, decay * S[r + 3]);
-      }
-      o0 = fmaf(S[r], q.x, o0);
-      o1 = fmaf(S[r + 1], q.y, o1);
-      o2 = fmaf(S[r + 2], q.z, o2);
-      o3 = fmaf(S[r + 3], q.w, o3);
+      S[2 * r4] = step(S[2 * r4], make_float2(a.x, a.y));
+      S[2 * r4 + 1] = step(S[2 * r4 + 1], make_float2(a.z, a.w));
+      o01 = fma2(S[2 * r4], make_float2(q.x, q.y), o01);
+      o23 = fma2(S[2 * r4 + 1], make_float2(q.z, q.w), o23);
     }
-    return (o0 + o1) + (o2 + o3);
+    return (o01.x + o01.y) + (o23.x + o23.y);
   };
   // a token's row of [q | a | v] in shared memory into registers
   auto fetch = [&](const float* row, float4 (&qs)[ROWS / 4], float4 (&as)[ROWS / 4], float& v, float& d) {
@@ -363,8 +362,180 @@ linear_scan_kernel(LinearScanParams p, int lanes, int slices) {
   }
   if (walker) {
 #pragma unroll
-    for (int r = 0; r < ROWS; ++r) mem[(int64_t)r * threads] = S[r];
+    for (int r = 0; r < ROWS; r += 2) {
+      mem[(int64_t)r * threads] = S[r / 2].x;
+      mem[(int64_t)(r + 1) * threads] = S[r / 2].y;
+    }
   }
+}
+
+// The prompt form for heads whose rows are whole 16-byte pieces.  What bounds the scan above is the way from shared memory
+// into registers (128 bytes a cycle and SM, broadcast or not): a thread reads 2 x ROWS numbers of q and a for ROWS elements
+// of S.  Here a thread owns QUADS quads of rows x 4 columns of S in pairs, so that 16 numbers (and four of v) serve 32
+// elements; RL lanes x 4 QUADS rows cover the dim, a block again 32 columns.  The outputs of two tokens, eight sums, go
+// through one exchange over RL lanes.  A token's numbers stand in registers one token ahead; tokens arrive kWalkChunk at a
+// time by asynchronous copies, a warp a token.  Forget gates, 16 heads of 128 x 128 (us, before | now, with the preparation):
+// one sequence of 2,048 tokens 394 | 326, two of 1,024 232 | 181, seven of 300 281 | 152; 32 heads 458 | 345, 464 | 269,
+// 509 | 251.
+constexpr int kWalkChunk = 16;
+template <int MODE, int RL, int QUADS>
+__global__ void __launch_bounds__(RL * 8) linear_walk_kernel(LinearScanParams p, int rows, int lanes, int slices) {
+  constexpr int kRowsPadded = RL * 4 * QUADS, kPairs = 2 * QUADS, kWarps = RL / 4;
+  constexpr int kToken = 2 * kRowsPadded + kScanColumns + (MODE == kTokenDecay ? 4 : 0);       // [q | a | v (| decay)]
+  constexpr int kPieces = (2 * kRowsPadded + kScanColumns + 127) / 128;
+  extern __shared__ __align__(16) float smem[];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int H = p.num_heads, D = p.head_dim, DV = p.v_dim;
+  const int slice = blockIdx.x % slices;
+  const int head = (blockIdx.x / slices) % H;
+  const int seq = blockIdx.x / (slices * H);
+  const int slot = p.state_slots[seq];
+  const int first = p.cu_q[seq];
+  const int n = p.cu_q[seq + 1] - first;
+  // a padded sequence: nothing is read or written (nor for rows that are not the batch's, or a slot that is not there)
+  if (slot < 0 || slot >= p.num_slots || n <= 0 || first < 0 || (int64_t)first + n > p.num_tokens) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int rl = lane % RL, col = (warp * (32 / RL) + lane / RL) * 4;
+  const int mine_cols = min(kScanColumns, DV - slice * kScanColumns);
+  const int qk_head = head / p.qk_group;
+  const float decay = (MODE == kConstantDecay || MODE == kPlainDecay) ? p.decay[head] : 0.f;
+  // row i of the thread's: 4 RL (i / 4) + 4 rl + i % 4, and where it lies in the state slot
+  float* memory = p.state + (int64_t)slot * p.state_stride + ((int64_t)head * slices + slice) * rows * kScanColumns * lanes;
+  auto place = [&](int i, int c) -> float* {
+    const int d = (i >> 2) * 4 * RL + 4 * rl + (i & 3);
+    return d < rows * lanes ? memory + ((int64_t)(d % rows) * kScanColumns + col + c) * lanes + d / rows : nullptr;
+  };
+  float2 S[kPairs][4];                                 // [pair of rows][column]
+#pragma unroll
+  for (int r = 0; r < kPairs; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float *a = place(2 * r, c), *b = place(2 * r + 1, c);
+      S[r][c] = make_float2(a != nullptr ? *a : 0.f, b != nullptr ? *b : 0.f);
+    }
+  int piece_from[kPieces], piece_to[kPieces];
+#pragma unroll
+  for (int r = 0; r < kPieces; ++r) {
+    const int i = (lane + 32 * r) * 4;
+    piece_to[r] = -1;
+    piece_from[r] = 0;
+    if (i < D) {
+      piece_from[r] = p.act_q_off + qk_head * D + i;
+      piece_to[r] = i;
+    } else if (i < 2 * D) {
+      piece_from[r] = p.act_k_off + qk_head * D + (i - D);
+      piece_to[r] = kRowsPadded + (i - D);
+    } else if (i < 2 * D + mine_cols) {
+      piece_from[r] = p.act_v_off + head * DV + slice * kScanColumns + (i - 2 * D);
+      piece_to[r] = 2 * kRowsPadded + (i - 2 * D);
+    }
+  }
+  auto copy = [&](float* buffer, int t0, int count) {
+    for (int t = warp; t < count; t += kWarps) {
+      const float* row = p.act + (int64_t)(first + t0 + t) * p.act_stride;
+#pragma unroll
+      for (int r = 0; r < kPieces; ++r)
+        if (piece_to[r] >= 0) copy_async<16>(buffer + t * kToken + piece_to[r], row + piece_from[r]);
+      if (MODE == kTokenDecay && lane == 0)
+        copy_async<4>(buffer + t * kToken + 2 * kRowsPadded + kScanColumns, row + p.decay_off + head);
+    }
+    copy_async_commit();
+  };
+  struct Token {
+    float2 q[kPairs], a[kPairs];
+    float4 v;
+    float decay;
+  };
+  // a lane ends an exchange with the sum of one column, of the first or (second) the second of two tokens
+  const bool second = spread_index<RL>(lane) >= 4;
+  const int own = col + (spread_index<RL>(lane) & 3);
+  const bool stores = rl % (RL / 8 > 0 ? RL / 8 : 1) == 0 && own < mine_cols;
+  auto load = [&](Token& x, const float* row) {
+#pragma unroll
+    for (int i = 0; i < QUADS; ++i) {
+      const float4 q = *reinterpret_cast<const float4*>(row + i * 4 * RL + 4 * rl);
+      const float4 a = *reinterpret_cast<const float4*>(row + kRowsPadded + i * 4 * RL + 4 * rl);
+      x.q[2 * i] = make_float2(q.x, q.y);
+      x.q[2 * i + 1] = make_float2(q.z, q.w);
+      x.a[2 * i] = make_float2(a.x, a.y);
+      x.a[2 * i + 1] = make_float2(a.z, a.w);
+    }
+    x.v = *reinterpret_cast<const float4*>(row + 2 * kRowsPadded + col);
+    x.decay = MODE == kTokenDecay ? row[2 * kRowsPadded + kScanColumns] : decay;
+  };
+  // token x applied to S; this lane's parts of its output
+  auto step = [&](const Token& x, float* parts) {
+    const float vs[4] = {x.v.x, x.v.y, x.v.z, x.v.w};
+    const float2 dd = make_float2(x.decay, x.decay);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float2 v = make_float2(vs[c], vs[c]), minus = make_float2(-vs[c], -vs[c]);
+      float2 sum;
+#pragma unroll
+      for (int r = 0; r < kPairs; ++r) {
+        // f S + (1 - f) v as v + f (S - v); the others k v + decay S
+        S[r][c] = MODE == kGatedWrite ? fma2(x.a[r], add2(S[r][c], minus), v) : fma2(x.a[r], v, mul2(dd, S[r][c]));
+        sum = r == 0 ? mul2(S[r][c], x.q[r]) : fma2(S[r][c], x.q[r], sum);
+      }
+      parts[c] = sum.x + sum.y;
+    }
+  };
+  auto put = [&](const float (&parts)[8], float* to, int64_t wide, bool both) {
+    const float o = spread_sum8<RL>(parts, lane);
+    if (stores && (both || !second)) to[(second ? wide : 0) + own] = o;
+  };
+  // rows of S beyond the dim never change: q and k stay zero there, a forget gate one; value columns beyond the width
+  // stay zero
+  for (int i = threadIdx.x; i < (2 * kWalkChunk + 1) * kToken; i += blockDim.x) {
+    const int e = i % kToken;
+    smem[i] = (MODE == kGatedWrite && e >= kRowsPadded && e < 2 * kRowsPadded) ? 1.f : 0.f;
+  }
+  __syncthreads();
+  copy(smem, 0, min(kWalkChunk, n));
+  copy_async_wait_all();
+  __syncthreads();
+  const int64_t wide = (int64_t)H * DV;
+  float* out = p.out + (int64_t)first * wide + (int64_t)head * DV + slice * kScanColumns;
+  for (int c0 = 0; c0 < n; c0 += kWalkChunk) {
+    const int count = min(kWalkChunk, n - c0), next = min(kWalkChunk, n - c0 - kWalkChunk);
+    const float* buffer = smem + ((c0 / kWalkChunk) & 1) * kWalkChunk * kToken;
+    if (next > 0) copy(smem + (((c0 / kWalkChunk) & 1) ^ 1) * kWalkChunk * kToken, c0 + kWalkChunk, next);
+    float* to = out + (int64_t)c0 * wide;
+    Token even, odd;
+    load(even, buffer);
+    if (count == kWalkChunk) {
+      // no branch between tokens, so that one's read-out can stand among the next one's instructions (the load behind the
+      // last token brings nothing that is used; there is room for it behind the second buffer)
+#pragma unroll 2
+      for (int t = 0; t < kWalkChunk; t += 2) {
+        float parts[8];
+        load(odd, buffer + (t + 1) * kToken);
+        step(even, parts);
+        load(even, buffer + (t + 2) * kToken);
+        step(odd, parts + 4);
+        put(parts, to + t * wide, wide, true);
+      }
+    } else {
+      for (int t = 0; t < count; ++t) {
+        float parts[8] = {};
+        load(odd, buffer + (t + 1) * kToken);
+        step(even, parts);
+        put(parts, to + t * wide, wide, false);
+        even = odd;
+      }
+    }
+    copy_async_wait_all();
+    __syncthreads();
+  }
+#pragma unroll
+  for (int r = 0; r < kPairs; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      float *a = place(2 * r, c), *b = place(2 * r + 1, c);
+      if (a != nullptr) *a = S[r][c].x;
+      if (b != nullptr) *b = S[r][c].y;
+    }
 }
 
 // v[t, c]   = in[t, c] (+ skip_coef[c / skip_head] * skip[t, skip_off + c])  (* gate(x[t, gate_off + c]), gate_first)
@@ -448,20 +619,49 @@ static int launch_scan_chunk(const LinearScanParams& p, int lanes, cudaStream_t 
                            dim3(1, 1, 1), p, lanes, slices);
 }
 
+template <int MODE, int RL, int QUADS>
+static int launch_walk(const LinearScanParams& p, int rows, int lanes, cudaStream_t stream) {
+  const int slices = (p.v_dim + kScanColumns - 1) / kScanColumns;
+  const int64_t blocks = (int64_t)p.num_seqs * p.num_heads * slices;
+  if (blocks > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
+  const size_t smem = (2 * (size_t)kWalkChunk + 1) * (2 * RL * 4 * QUADS + kScanColumns + (MODE == kTokenDecay ? 4 : 0)) * sizeof(float);
+  auto kernel = linear_walk_kernel<MODE, RL, QUADS>;
+  if (smem > 48 * 1024) {
+    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err != cudaSuccess) return (int)err;
+  }
+  return (int)launch_alone(kernel, dim3((unsigned)blocks), dim3(RL * 8), smem, stream, p, rows, lanes, slices);
+}
+
 // Steps of about a token per sequence (decoding; the caller gives no scratch) stage two tokens at a time, every
 // thread its share: few registers and little shared memory per block, so more blocks share an SM while the memories
-// stream through.  Other steps have their activations and gates worked out by a kernel of its own, and the scan
-// stages 32 tokens (eight where a lane holds 32 rows) by asynchronous copies in warps of their own.
+// stream through.  Other steps have their activations and gates worked out by a kernel of its own and walk in register
+// tiles where all rows are whole 16-byte pieces; otherwise the scan stages 32 tokens (eight where a lane holds 32 rows)
+// number by number in warps of their own.
 template <typename T, int MODE, int ROWS>
 static int launch_scan(const LinearScanParams& p, int lanes, cudaStream_t stream) {
   if (p.act == nullptr) return launch_scan_chunk<T, MODE, ROWS, 2, 0>(p, lanes, stream);
   if (p.num_tokens > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
   if constexpr (MODE == kGatedWrite || MODE == kConstantDecay) {
     const int width = 2 * p.num_heads * p.head_dim + p.num_heads * p.v_dim;
-    const int across = std::min((width + 255) / 256, 64);
-    const int err = (int)launch_chain(linear_prep_kernel<T, MODE>, dim3((unsigned)p.num_tokens, (unsigned)across),
-                                      dim3(256), 0, stream, dim3(1, 1, 1), p, width);
+    const int qk = p.num_heads * p.head_dim;
+    const bool fours = qk % 4 == 0 && width % 4 == 0 && p.x_stride % 4 == 0 && p.q_off % 4 == 0 && p.k_off % 4 == 0 &&
+                       p.v_off % 4 == 0 && reinterpret_cast<uintptr_t>(p.x) % (4 * sizeof(T)) == 0 &&
+                       (reinterpret_cast<uintptr_t>(p.act) | reinterpret_cast<uintptr_t>(p.lower) |
+                        reinterpret_cast<uintptr_t>(p.gate_bias)) % 16 == 0;
+    const int across = std::min((width + 256 * (fours ? 4 : 1) - 1) / (256 * (fours ? 4 : 1)), 64);
+    const dim3 grid((unsigned)p.num_tokens, (unsigned)across);
+    const int err = (int)(fours ? launch_chain(linear_prep_kernel<T, MODE, 4>, grid, dim3(256), 0, stream, dim3(1, 1, 1), p, width)
+                                : launch_chain(linear_prep_kernel<T, MODE, 1>, grid, dim3(256), 0, stream, dim3(1, 1, 1), p, width));
     if (err != 0) return err;
+  }
+  if (p.head_dim % 4 == 0 && p.v_dim % 4 == 0 && p.act_aligned) {
+    if constexpr (ROWS == 16) {
+      if (p.head_dim <= 64) return launch_walk<MODE, 8, 2>(p, ROWS, lanes, stream);
+      return launch_walk<MODE, 16, 2>(p, ROWS, lanes, stream);
+    } else {
+      return launch_walk<MODE, 32, 2>(p, ROWS, lanes, stream);
+    }
   }
   return launch_scan_chunk<T, MODE, ROWS, (ROWS >= 32 ? 8 : 32), kScanProducers>(p, lanes, stream);
 }
@@ -493,7 +693,7 @@ int launch_linear_scan(const LinearScanParams& given, cudaStream_t stream) {
     p.act_q_off = 0;
     p.act_k_off = qk;
     p.act_v_off = 2 * qk;
-    p.act_aligned = 1;
+    p.act_aligned = (p.act_stride % 4 == 0 && reinterpret_cast<uintptr_t>(p.act) % 16 == 0) ? 1 : 0;
   }
   int rows = 0, lanes = 0;
   if (!linear_scan_shape(p.head_dim, p.v_dim, &rows, &lanes) || p.num_heads < 1 || p.mode < kGatedWrite ||
