@@ -430,10 +430,11 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __grid
     // inside the sigmoid, in log2 units
     const float head_bias = (sigmoid && fp.head_bias != nullptr) ? fp.head_bias[kvh * G + head_local] * kLog2e : 0.f;
     float m_ref = -CUDART_INF_F, l = 0.f;
-    // a sink: the walk starts as if a key of that score and of value zero had come first
+    // a sink: the walk starts as if a key of that score and of value zero had come first (a score of minus infinity
+    // counts nothing: the first block would raise it without a factor that could take the 1 out again)
     if (kScored && fp.sink != nullptr && live) {
       m_ref = fp.sink[kvh * G + head_local] * kLog2e;
-      l = 1.f;
+      l = m_ref > -CUDART_INF_F ? 1.f : 0.f;
     }
 
     for (int b = 0; b < num_blocks; ++b) {

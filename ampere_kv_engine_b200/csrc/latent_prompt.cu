@@ -280,9 +280,10 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
     const float scale_log2 = p.scale * kLog2e;
     float m_ref = -CUDART_INF_F, l = 0.f;              // l: this half's share of the row sum
     if (p.sink != nullptr && live) {
-      // the walk starts as if a key of that score and of value zero had come first; one half counts it
+      // the walk starts as if a key of that score and of value zero had come first; one half counts it (a score of minus
+      // infinity counts nothing: the first block would raise it without a factor that could take the 1 out again)
       m_ref = p.sink[head] * kLog2e;
-      l = half == 0 ? 1.f : 0.f;
+      l = half == 0 && m_ref > -CUDART_INF_F ? 1.f : 0.f;
     }
     for (int b = 0; b < num_blocks; ++b) {
       const int key0 = key_begin + b * kKeys + half * 64;      // this thread's first key of the block
