@@ -822,13 +822,14 @@ void scored_attention(const Tensor& q, const Tensor& k_cache, const Tensor& v_ca
 
 // out[r] = the cache row of the plan's r-th key, zeros behind a sequence's context (launchers.h describes the plan).
 void latent_gather(const Tensor& cache, const Tensor& block_table, const Tensor& plan, Tensor& out, int64_t num_seqs,
-                   const OptTensor& status) {
+                   int64_t rank, const OptTensor& status) {
   check_cuda(cache, "cache");
   check_cuda(out, "out");
   check_same(cache, out, "cache", "out");
   AKV_CHECK(cache.scalar_type() == at::kBFloat16 && cache.dim() == 4 && cache.size(1) == 1 && out.dim() == 2 &&
                 out.size(1) == cache.size(3) && cache.size(3) % 8 == 0,
             "latent_gather: bfloat16 cache [pages, 1, page size, width], out [rows, width], a width of whole 16-byte pieces");
+  AKV_CHECK(rank >= 8 && rank % 8 == 0 && rank < cache.size(3), "latent_gather: rank is a multiple of 8 below the width");
   check_i32(block_table, "block_table");
   AKV_CHECK(block_table.dim() == 2, "block_table must be [sequences, width]");
   check_i32(plan, "plan");
@@ -844,6 +845,7 @@ void latent_gather(const Tensor& cache, const Tensor& block_table, const Tensor&
   p.page_size = (int)cache.size(2);
   p.table_width = (int)block_table.size(1);
   p.width = (int)cache.size(3);
+  p.rank = (int)rank;
   p.status = status_ptr(status);
   c10::cuda::CUDAGuard guard(cache.device());
   check_launch(akv::launch_latent_gather(p, stream_of(cache)), "latent_gather");
@@ -2480,7 +2482,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("out"), py::arg("status") = py::none());
   m.def("scaled_sum", &scaled_sum, py::arg("a"), py::arg("b"), py::arg("out"), py::arg("sa"), py::arg("sb"));
   m.def("latent_gather", &latent_gather, py::arg("cache"), py::arg("block_table"), py::arg("plan"), py::arg("out"),
-        py::arg("num_seqs"), py::arg("status") = py::none());
+        py::arg("num_seqs"), py::arg("rank"), py::arg("status") = py::none());
   m.def("latent_prompt_attention", &latent_prompt_attention, py::arg("q"), py::arg("q_rows"), py::arg("kv"),
         py::arg("latents"), py::arg("out"), py::arg("plan"), py::arg("num_seqs"), py::arg("num_tiles"), py::arg("heads"),
         py::arg("dim"), py::arg("rot_dim"), py::arg("v_dim"), py::arg("rank"), py::arg("window"), py::arg("scale"),

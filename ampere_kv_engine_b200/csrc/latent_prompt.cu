@@ -109,12 +109,19 @@ __device__ __forceinline__ void tmem_store16(uint32_t taddr, const uint32_t (&r)
       : "memory");
 }
 __device__ __forceinline__ void tmem_wait_store() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// whether neither of two packed bfloat16 numbers is infinite or NaN (an exponent of all ones)
+__device__ __forceinline__ bool both_finite(uint32_t w) {
+  return (w & 0x7f80u) != 0x7f80u && (w & 0x7f800000u) != 0x7f800000u;
+}
 __device__ __forceinline__ void pair_sync(int id) { asm volatile("barrier.cta.sync %0, 64;" ::"r"(id) : "memory"); }
 
 }  // namespace
 
 // A warp per gathered row.  Row r belongs to the last sequence of the plan whose first row is not behind r and holds its
 // key first_key + (r - first row), zeros from the context's end on.
+// A row whose latent is not finite gets zeros for it and NaN for its turned part: its score is then NaN for every query
+// that sees it, and its value is finite, so that P V (0 times the value where a row of the tile does not see the key)
+// leaves the other rows of a 128-row tile alone.
 __global__ void __launch_bounds__(256) latent_gather_kernel(LatentGatherParams p) {
   pdl_launch_dependents();
   pdl_wait();
@@ -140,13 +147,22 @@ __global__ void __launch_bounds__(256) latent_gather_kernel(LatentGatherParams p
     }
   }
   uint4* dst = reinterpret_cast<uint4*>((__nv_bfloat16*)p.out + r * p.width);
-  for (int c = lane; c < p.width / 8; c += 32) dst[c] = src != nullptr ? src[c] : make_uint4(0u, 0u, 0u, 0u);
+  bool finite = true;
+  for (int c = lane; c < p.width / 8; c += 32) {
+    const uint4 v = src != nullptr ? src[c] : make_uint4(0u, 0u, 0u, 0u);
+    if (c < p.rank / 8) finite = finite && both_finite(v.x) && both_finite(v.y) && both_finite(v.z) && both_finite(v.w);
+    dst[c] = v;
+  }
+  if (!__all_sync(0xffffffffu, finite)) {
+    const uint4 nan = make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
+    for (int c = lane; c < p.width / 8; c += 32) dst[c] = c < p.rank / 8 ? make_uint4(0u, 0u, 0u, 0u) : nan;
+  }
 }
 
 int launch_latent_gather(const LatentGatherParams& p, cudaStream_t stream) {
   if (p.rows == 0) return 0;
   const int64_t blocks = (p.rows + 7) / 8;
-  if (p.num_seqs < 1 || p.width % 8 || blocks > 0x7fffffffLL || reinterpret_cast<uintptr_t>(p.cache) % 16 ||
+  if (p.num_seqs < 1 || p.width % 8 || p.rank % 8 || p.rank >= p.width || blocks > 0x7fffffffLL || reinterpret_cast<uintptr_t>(p.cache) % 16 ||
       reinterpret_cast<uintptr_t>(p.out) % 16)
     return (int)cudaErrorInvalidValue;
   return (int)launch_chain(latent_gather_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, dim3(1, 1, 1), p);

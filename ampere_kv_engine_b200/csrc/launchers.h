@@ -267,6 +267,7 @@ struct LatentGatherParams {
   void* out;                   // [rows, width]
   int64_t rows, num_pages;
   int num_seqs, page_size, table_width, width;
+  int rank;                    // the row's first columns, its latent; the rest is its turned part
   int* status;
 };
 int launch_latent_gather(const LatentGatherParams& p, cudaStream_t stream);

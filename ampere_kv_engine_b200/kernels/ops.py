@@ -554,7 +554,7 @@ def latent_prompt_attention(q, q_rows, cache, block_table, plan: LatentPlan, w_k
     head; ``q_rows`` [tokens, heads * (rank + rot_dim)]: the turned ones behind the first ``rank`` columns.  Writes the
     portions' rows of ``out`` [tokens, heads * v_dim]; ``gate`` and ``sink`` as for :func:`scored_attention`."""
     latents = torch.empty((plan.rows, rank + rot_dim), dtype=cache.dtype, device=cache.device)
-    ext().latent_gather(cache, block_table, plan.plan, latents, plan.num_seqs, status)
+    ext().latent_gather(cache, block_table, plan.plan, latents, plan.num_seqs, rank, status)
     kv = torch.nn.functional.linear(latents[:, :rank], w_kv)
     ext().latent_prompt_attention(q, q_rows, kv, latents, out, plan.plan, plan.num_seqs, plan.num_tiles, heads, dim, rot_dim,
                                   v_dim, rank, int(window or 0), float(scale), gate, sink, status)
