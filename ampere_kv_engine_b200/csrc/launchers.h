@@ -460,9 +460,9 @@ struct MoeGemmParams {
   int activation;              // up: an Activation
   int* status;                 // kernels' status word, or null
 };
-// steps with at most this many (token, choice) pairs that the tcgen05 form does not take run the few-rows form of the
-// gated product (against mma.sync tiles at 8 tokens, 64 experts of 1,024 x 4,096: 103 against 111 us; the down product
-// is faster in tiles: 59 against 89 us)
+// most (token, choice) pairs that the few-rows form takes by itself: first products of hidden sizes below the tcgen05
+// form's K block (against mma.sync tiles at 8 tokens, 64 experts of 1,024 x 4,096: 103 against 111 us; the down product
+// is faster in tiles: 59 against 89 us), and those of experts without a gate on a few tokens (launch_moe_form)
 constexpr int kMoeFewRowPairs = 128;
 int launch_moe_gemm(const MoeGemmParams& p, MoeForm form, cudaStream_t stream);
 bool moe_gemm_takes_tc(const MoeGemmParams& p, MoeForm form);

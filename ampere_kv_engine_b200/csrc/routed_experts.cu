@@ -707,13 +707,20 @@ __global__ void __launch_bounds__(kGemvWarps * 32) moe_gemv_kernel(MoeGemmParams
 namespace {
 template <int FORM>
 int launch_moe_form(const MoeGemmParams& p, cudaStream_t stream) {
-  // 0: by size; 1: float arithmetic; 2: mma.sync tiles; 3: the few-rows form; 4: tcgen05 tiles.  Whatever the tcgen05
-  // form takes it is the fastest at every size measured (us, gated / down product, 64 experts of 1,024 x 4,096 with 6
-  // choices, tcgen05 | mma.sync tiles | few rows): 1 token 43 / 22 | 81 / 33 | 62 / 29; 8 tokens 103 / 55 | 123 / 68 |
-  // 115 / 68; 64 tokens 195 / 109 | 275 / 143 | 470 / 224; 2,048 tokens 282 / 185 | 881 / 520.  The other two serve
-  // hidden sizes below one K block of 64.
+  // 0: by size; 1: float arithmetic; 2: mma.sync tiles; 3: the few-rows form; 4: tcgen05 tiles.  The tcgen05 form is the
+  // fastest of all that it takes (us, gated / down product, 64 experts of 1,024 x 4,096 with 6 choices, tcgen05 |
+  // mma.sync tiles | few rows: 1 token 43 / 22 | 81 / 33 | 62 / 29; 8 tokens 103 / 55 | 123 / 68 | 115 / 68; 64 tokens
+  // 195 / 109 | 275 / 143 | 470 / 224; 2,048 tokens 282 / 185 | 881 / 520) but for one product: the first one of experts
+  // without a gate on a few tokens.  A tcgen05 tile takes 256 features there, so a token's choices fill a handful of
+  // SMs, each with the whole K in a row; the few-rows form spreads them over all (K = 2,048, cold weights, tcgen05 | few
+  // rows: 4 choices of 768 features 22.6 | 14.1, 16 choices 22.9 | 16.6; K = 4,096, 12 choices of 1,024 40.7 | 29.4).  It
+  // wins while its blocks of 32 features run in one round (384 blocks; 576 took 28.7 against 23.1) and an expert's rows
+  // are at most two of its passes (8 tokens that all choose the same experts 22 | 25, 12 tokens 26 | 27 to 52 | 44).
+  // The mma.sync tiles, and the few-rows form otherwise, serve hidden sizes below one K block of 64.
+  const bool few_blocks = FORM == kMoeUp && p.pairs <= kMoeFewRowPairs && p.pairs <= (int64_t)p.top * 2 * kGemvRows &&
+                          p.pairs * ((p.n + kGemvFeatures - 1) / kGemvFeatures) <= 384;
   const bool tensor_ok = moe_gemm_takes_mma(p);
-  if (p.force_plain == 4 || (p.force_plain == 0 && moe_gemm_takes_tc(p, (MoeForm)FORM)))
+  if (p.force_plain == 4 || (p.force_plain == 0 && !(few_blocks && tensor_ok) && moe_gemm_takes_tc(p, (MoeForm)FORM)))
     return launch_moe_gemm_tc(p, (MoeForm)FORM, stream);
   if ((p.force_plain == 2 || p.force_plain == 3) && !tensor_ok) return (int)cudaErrorInvalidValue;
   if (p.force_plain == 3 || (p.force_plain == 0 && tensor_ok && FORM != kMoeDown && p.pairs <= kMoeFewRowPairs)) {

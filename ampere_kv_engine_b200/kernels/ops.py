@@ -756,7 +756,8 @@ def moe_gate_up(x, w_gate_up, order, offsets, *, top, limit, slope, kernel: str 
 def moe_up(x, w_up, order, offsets, *, top, activation: str, kernel: str = "auto", status=None):
     """Row r of the result belongs to pair ``order[r]`` and is ``activation(W_up x)`` of its expert (one without a gate)
     for the pair's token; ``w_up`` [experts, intermediate, hidden].  [tokens * top, intermediate] in the dtype of ``x``.
-    ``kernel`` as for :func:`moe_gate_up`."""
+    ``kernel`` as for :func:`moe_gate_up`, but that ``"auto"`` takes the few-rows form for up to eight tokens whose pairs
+    times features (in 32s) come to at most 384."""
     act = torch.empty((order.numel(), w_up.shape[1]), dtype=x.dtype, device=x.device)
     ext().moe_up(x, w_up, order, offsets, act, top, ACTIVATIONS[activation], MOE_FORMS[kernel],
                  **_status_of(status, x))
