@@ -1386,7 +1386,7 @@ void delta_scan(const Tensor& qkv, const Tensor& coef, const Tensor& x, const Te
                 const Tensor& cu_q, const Tensor& state_slots, Tensor& scratch, Tensor& out, int64_t num_heads,
                 int64_t num_kv_heads, int64_t head_dim, int64_t v_dim, int64_t taps, double norm_eps,
                 const OptTensor& gates, int64_t gate_off, int64_t gate_kind, bool channel_decay, int64_t x_off,
-                int64_t out_off, double factor) {
+                int64_t out_off, double factor, const OptTensor& status) {
   akv::DeltaParams p = delta_params(x, state, cu_q, state_slots, num_heads, num_kv_heads, head_dim, v_dim, taps, x_off,
                                     !gates.has_value());
   const int64_t channels = 2 * num_kv_heads * head_dim + num_heads * v_dim;
@@ -1421,6 +1421,7 @@ void delta_scan(const Tensor& qkv, const Tensor& coef, const Tensor& x, const Te
   p.out_off = (int)out_off;
   p.factor = (float)factor;
   p.norm_eps = (float)norm_eps;
+  p.status = status_ptr(status);
   c10::cuda::CUDAGuard guard(x.device());
   check_launch(akv::launch_delta_scan(p, stream_of(x)), "delta_scan");
 }
@@ -1430,7 +1431,7 @@ void delta_scan(const Tensor& qkv, const Tensor& coef, const Tensor& x, const Te
 void linear_scan(const Tensor& x, Tensor& state, const Tensor& cu_q, const Tensor& state_slots, Tensor& out,
                  int64_t num_heads, int64_t head_dim, int64_t v_dim, int64_t mode, int64_t q_off, int64_t k_off,
                  int64_t v_off, const OptTensor& gate_bias, const OptTensor& lower, const OptTensor& decay,
-                 int64_t qk_group, int64_t decay_off) {
+                 int64_t qk_group, int64_t decay_off, const OptTensor& status) {
   check_cuda(x, "x");
   AKV_CHECK(x.dim() == 2, "x must be [tokens, columns]");
   AKV_CHECK(num_heads > 0 && akv::linear_scan_state_floats((int)num_heads, (int)head_dim, (int)v_dim) > 0,
@@ -1500,6 +1501,7 @@ void linear_scan(const Tensor& x, Tensor& state, const Tensor& cu_q, const Tenso
   p.v_dim = (int)v_dim;
   p.mode = (int)mode;
   p.dtype = dtype_code(x, "x");
+  p.status = status_ptr(status);
   c10::cuda::CUDAGuard guard(x.device());
   check_launch(akv::launch_linear_scan(p, stream_of(x)), "linear_scan");
 }
@@ -1892,6 +1894,7 @@ void conv_tail(const Tensor& x, Tensor& state, int64_t tail_off, const Tensor& c
     check_f32(*bias, "bias", channels);
     p.bias = bias->data_ptr<float>();
   }
+  p.num_tokens = x.size(0);
   p.x_stride = x.size(1);
   p.conv_off = (int)conv_off;
   p.channels = (int)channels;
@@ -2422,7 +2425,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("cu_q"), py::arg("state_slots"), py::arg("scratch"), py::arg("out"), py::arg("num_heads"),
         py::arg("num_kv_heads"), py::arg("head_dim"), py::arg("v_dim"), py::arg("taps"), py::arg("norm_eps"),
         py::arg("gates") = py::none(), py::arg("gate_off") = 0, py::arg("gate_kind") = 0, py::arg("channel_decay") = false,
-        py::arg("x_off") = 0, py::arg("out_off") = 0, py::arg("factor") = 1.0);
+        py::arg("x_off") = 0, py::arg("out_off") = 0, py::arg("factor") = 1.0, py::arg("status") = py::none());
   m.def("delta_scan_supported", [](int64_t dim, int64_t v_dim) { return akv::delta_scan_supported((int)dim, (int)v_dim); });
   m.def("delta_memory_floats", [](int64_t heads, int64_t dim, int64_t v_dim) {
     return akv::delta_memory_floats((int)heads, (int)dim, (int)v_dim);
@@ -2430,7 +2433,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("linear_scan", &linear_scan, py::arg("x"), py::arg("state"), py::arg("cu_q"), py::arg("state_slots"),
         py::arg("out"), py::arg("num_heads"), py::arg("head_dim"), py::arg("v_dim"), py::arg("mode"), py::arg("q_off"),
         py::arg("k_off"), py::arg("v_off"), py::arg("gate_bias") = py::none(), py::arg("lower") = py::none(),
-        py::arg("decay") = py::none(), py::arg("qk_group") = 1, py::arg("decay_off") = 0);
+        py::arg("decay") = py::none(), py::arg("qk_group") = 1, py::arg("decay_off") = 0, py::arg("status") = py::none());
   m.def("linear_scan_state_floats", [](int64_t heads, int64_t dim, int64_t v_dim) {
     return (int64_t)akv::linear_scan_state_floats((int)heads, (int)dim, (int)v_dim);
   });

@@ -18,14 +18,24 @@ enum DType : int { kFloat32 = 0, kBFloat16 = 1 };
 enum Status : int {
   kOk = 0,
   kBadPage = 1,      // a block-table entry outside [0, num_pages)
-  kBadSlot = 2,      // a cache slot outside the pool
+  kBadSlot = 2,      // a cache slot outside the pool, or a state slot outside the state
   kBadToken = 3,     // a token id outside the vocabulary
-  kBadRow = 4,       // a gathered row outside the batch
+  kBadRow = 4,       // a gathered row, or a row of a sequence, outside the batch
   kWaitTimeout = 5,  // a bounded mbarrier wait gave up
 };
 
 __device__ __forceinline__ void set_status(int* status, int code) {
   if (status != nullptr) atomicCAS(status, 0, code);
+}
+
+// Whether a sequence's rows [first, first + n) lie in the batch and its state slot below the state's end.  What does not
+// is reported by the block's first thread, and the caller must not follow it.
+__device__ __forceinline__ bool sequence_inside(int64_t first, int64_t n, int64_t num_tokens, int slot, int num_slots,
+                                                int* status) {
+  const bool rows = first >= 0 && n >= 0 && first + n <= num_tokens;
+  if (rows && slot < num_slots) return true;
+  if (threadIdx.x == 0) set_status(status, rows ? kBadSlot : kBadRow);
+  return false;
 }
 
 template <typename T>

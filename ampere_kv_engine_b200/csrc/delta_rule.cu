@@ -229,6 +229,14 @@ int64_t delta_memory_floats(int num_heads, int dim, int v_dim) {
   return (int64_t)num_heads * v_dim * s.lanes * s.ept;
 }
 
+// The output rows of a sequence that has no state or cannot be walked: zeros, those of them that are rows of the batch.
+static __device__ void zero_rows(const DeltaParams& p, int head, int col0, int cols, int64_t first, int64_t last) {
+  const int64_t begin = first > 0 ? first : 0, end = last < p.num_tokens ? last : p.num_tokens;
+  float* out = p.scratch + (int64_t)head * p.v_dim + col0;
+  for (int64_t i = threadIdx.x; i < (end - begin) * cols; i += blockDim.x)
+    out[(begin + i / cols) * p.num_heads * p.v_dim + i % cols] = 0.f;
+}
+
 template <int EPT, int LANES, int CHUNK, bool CHANNEL>
 __global__ void __launch_bounds__(256) delta_scan_kernel(DeltaParams p, int cols) {
   constexpr int kRounds = scan_rounds(EPT, CHANNEL);
@@ -244,11 +252,11 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(DeltaParams p, int cols
   const int64_t first = p.cu_q[s];
   const int n = (int)(p.cu_q[s + 1] - first);
   const int slot = p.state_slots[s];
-  if (n <= 0) return;
+  if (n == 0) return;
   const int mine_cols = min(cols, V - col0);
   float* scratch = p.scratch + first * H * V + (int64_t)h * V + col0;
-  if (slot < 0 || slot >= p.num_slots) {
-    for (int i = threadIdx.x; i < n * mine_cols; i += blockDim.x) scratch[(int64_t)(i / mine_cols) * H * V + i % mine_cols] = 0.f;
+  if (!sequence_inside(first, p.cu_q[s + 1] - first, p.num_tokens, slot, p.num_slots, p.status) || slot < 0) {
+    zero_rows(p, h, col0, mine_cols, first, p.cu_q[s + 1]);
     return;
   }
   float* state = p.state + (int64_t)slot * p.state_stride;
@@ -425,11 +433,11 @@ __global__ void __launch_bounds__(RL * 8) delta_walk_kernel(DeltaParams p, int e
   const int64_t first = p.cu_q[s];
   const int n = (int)(p.cu_q[s + 1] - first);
   const int slot = p.state_slots[s];
-  if (n <= 0 || first < 0 || first + n > p.num_tokens) return;
+  if (n == 0) return;
   const int mine_cols = min(kWalkColumns, V - col0);
   float* scratch = p.scratch + first * H * V + (int64_t)h * V + col0;
-  if (slot < 0 || slot >= p.num_slots) {
-    for (int i = threadIdx.x; i < n * mine_cols; i += blockDim.x) scratch[(int64_t)(i / mine_cols) * H * V + i % mine_cols] = 0.f;
+  if (!sequence_inside(first, p.cu_q[s + 1] - first, p.num_tokens, slot, p.num_slots, p.status) || slot < 0) {
+    zero_rows(p, h, col0, mine_cols, first, p.cu_q[s + 1]);
     return;
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -655,7 +663,7 @@ __global__ void __launch_bounds__(128) delta_finish_kernel(DeltaParams p, int no
   const int64_t first = p.cu_q[s];
   const int n = (int)(p.cu_q[s + 1] - first);
   const int slot = p.state_slots[s];
-  if (c >= channels || n <= 0 || slot < 0 || slot >= p.num_slots) return;
+  if (c >= channels || n <= 0 || slot < 0 || slot >= p.num_slots || first < 0 || first + n > p.num_tokens) return;
   const int keep = p.taps - 1;
   float* before = p.state + (int64_t)slot * p.state_stride + p.memory;
   float kept[kDeltaMaxTaps - 1];

@@ -413,6 +413,7 @@ struct DeltaParams {
   int gate_kind;               // 0: SiLU, 1: sigmoid
   int channel_decay;           // 1: a decay per head and key channel
   float factor;                // on the normed, gated output
+  int* status;                 // kernels' status word, or null
 };
 int launch_delta_prep(const DeltaParams& p, cudaStream_t stream);
 int launch_delta_scan(const DeltaParams& p, cudaStream_t stream);
@@ -520,6 +521,7 @@ struct LinearScanParams {
   int num_slots;               // rows of `state`
   int qk_group;                // heads that share one q and one k (0 or 1: every head its own)
   int decay_off;               // kTokenDecay: column of x where the token's decays (a float per head) begin
+  int* status;                 // kernels' status word, or null
   // filled in by the launcher: where the prompt form's staging warps find q, k and v in `act`
   int64_t act_stride;
   int act_q_off, act_k_off, act_v_off, act_aligned;
@@ -651,6 +653,7 @@ struct ConvTailParams {
   int64_t state_stride, tail_off;
   const int32_t* cu_q;
   const int32_t* state_slots;
+  int64_t num_tokens;
   int num_seqs, num_slots, dtype;
 };
 int launch_conv_tail(const ConvTailParams& p, cudaStream_t stream);

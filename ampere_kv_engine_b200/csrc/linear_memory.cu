@@ -111,6 +111,15 @@ __global__ void __launch_bounds__(256) linear_prep_kernel(LinearScanParams p, in
   }
 }
 
+// The output rows of a sequence that cannot be walked: zeros, those of them that are rows of the batch.
+__device__ void zero_rows(const LinearScanParams& p, int head, int slice, int64_t first, int64_t last) {
+  const int cols = min(kScanColumns, p.v_dim - slice * kScanColumns);
+  const int64_t begin = first > 0 ? first : 0, end = last < p.num_tokens ? last : p.num_tokens;
+  float* out = p.out + (int64_t)head * p.v_dim + slice * kScanColumns;
+  for (int64_t i = threadIdx.x; i < (end - begin) * cols; i += blockDim.x)
+    out[(begin + i / cols) * p.num_heads * p.v_dim + i % cols] = 0.f;
+}
+
 // PRODUCERS == 0: the decode form.  PRODUCERS > 0: the prompt form with that many further threads that only copy
 // the next chunk from p.act into shared memory beside the walk of the current one.
 template <typename T, int MODE, int ROWS, int CHUNK, int PRODUCERS>
@@ -129,7 +138,11 @@ linear_scan_kernel(LinearScanParams p, int lanes, int slices) {
   const int slot = p.state_slots[seq];
   const int t0 = p.cu_q[seq];
   const int n = p.cu_q[seq + 1] - t0;
-  if (slot < 0 || n <= 0) return;                      // a padded sequence: nothing is read or written
+  if (slot < 0 || n == 0) return;                      // a padded sequence: nothing is read or written
+  if (!sequence_inside(t0, (int64_t)p.cu_q[seq + 1] - t0, p.num_tokens, slot, p.num_slots, p.status)) {
+    zero_rows(p, head, slice, t0, p.cu_q[seq + 1]);
+    return;
+  }
   const int tid = threadIdx.x;
   const int threads = kScanColumns * lanes;            // threads that own rows of S
   const bool walker = tid < threads;
@@ -393,8 +406,11 @@ __global__ void __launch_bounds__(RL * 8) linear_walk_kernel(LinearScanParams p,
   const int slot = p.state_slots[seq];
   const int first = p.cu_q[seq];
   const int n = p.cu_q[seq + 1] - first;
-  // a padded sequence: nothing is read or written (nor for rows that are not the batch's, or a slot that is not there)
-  if (slot < 0 || slot >= p.num_slots || n <= 0 || first < 0 || (int64_t)first + n > p.num_tokens) return;
+  if (slot < 0 || n == 0) return;                      // a padded sequence: nothing is read or written
+  if (!sequence_inside(first, (int64_t)p.cu_q[seq + 1] - first, p.num_tokens, slot, p.num_slots, p.status)) {
+    zero_rows(p, head, slice, first, p.cu_q[seq + 1]);
+    return;
+  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int rl = lane % RL, col = (warp * (32 / RL) + lane / RL) * 4;
   const int mine_cols = min(kScanColumns, DV - slice * kScanColumns);

@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(128) conv_tail_kernel(ConvTailParams p, int ch
   const int64_t first = p.cu_q[s];
   const int n = (int)(p.cu_q[s + 1] - first);
   const int slot = p.state_slots[s];
-  if (c >= p.channels || n <= 0 || slot < 0 || slot >= p.num_slots) return;
+  if (c >= p.channels || n <= 0 || slot < 0 || slot >= p.num_slots || first < 0 || first + n > p.num_tokens) return;
   const int keep = p.taps - 1;
   const T* x = (const T*)p.x;
   const float bias = p.bias != nullptr ? p.bias[c] : 0.f;

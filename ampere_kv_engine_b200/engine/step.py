@@ -20,9 +20,9 @@ from .batch import BatchLayout, SeqStep, build_context, fill_host, make_context,
 
 _STATUS_TEXT = {
     1: "a block-table entry pointed outside the page pool",
-    2: "a cache slot was outside the page pool",
+    2: "a cache slot was outside the page pool, or a state slot outside the state",
     3: "a token id was outside the vocabulary",
-    4: "a wanted row was outside the batch",
+    4: "a wanted row, or a row of a sequence, was outside the batch",
     5: "a bounded wait inside a kernel gave up",
 }
 

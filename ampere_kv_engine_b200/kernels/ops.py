@@ -657,7 +657,7 @@ DELTA_GATES = {"silu": 0, "sigmoid": 1}
 
 def delta_scan(qkv, coef, x, norm_weight, state, cu_q, state_slots, *, num_heads, num_kv_heads, head_dim, v_dim, taps,
                norm_eps, gates=None, gate_off: int = 0, gate: str = "silu", channel_decay: bool = False, x_off: int = 0,
-               factor: float = 1.0, out=None, out_off: int = 0):
+               factor: float = 1.0, out=None, out_off: int = 0, status=None):
     """The recurrence over the step's tokens, sequence by sequence and head by head, from and into ``state``
     [slots, delta_state_floats(...)[1]] float32: ``S *= decay; u = beta (v - S^T k);
     S += k u^T; o = S^T q``; then ``o / sqrt(mean(o^2) + norm_eps) * norm_weight * silu(gate)`` with the gate columns
@@ -665,7 +665,7 @@ def delta_scan(qkv, coef, x, norm_weight, state, cu_q, state_slots, *, num_heads
     With ``gates`` (a product of its own) the gate columns stand there from ``gate_off`` on and ``x`` holds [q | k | v]
     from ``x_off``; ``gate`` names the gate's function; ``channel_decay``: every row of S has its own decay; the result
     is multiplied by ``factor``.  Returns [tokens, heads * v_dim] in the dtype of ``x``; with ``out`` (a wider matrix)
-    it is written to that one's columns from ``out_off`` on."""
+    it is written to that one's columns from ``out_off`` on.  ``status`` as for :func:`linear_scan`."""
     if out is None:
         out, out_off = torch.empty((x.shape[0], num_heads * v_dim), dtype=x.dtype, device=x.device), 0
     scratch = torch.empty((x.shape[0], num_heads * v_dim), dtype=torch.float32, device=x.device)
@@ -674,7 +674,7 @@ def delta_scan(qkv, coef, x, norm_weight, state, cu_q, state_slots, *, num_heads
         extra = dict(gates=gates, gate_off=int(gate_off), gate_kind=DELTA_GATES[gate], channel_decay=bool(channel_decay),
                      x_off=int(x_off), out_off=int(out_off), factor=float(factor))
     ext().delta_scan(qkv, coef, x, norm_weight, state, cu_q, state_slots, scratch, out, num_heads, num_kv_heads,
-                     head_dim, v_dim, taps, float(norm_eps), **extra)
+                     head_dim, v_dim, taps, float(norm_eps), **extra, **_status_of(status, x))
     _launched(2)        # the scan; the output norm and the convolutions' memory
     return out
 
@@ -732,7 +732,7 @@ def moe_sort(chosen, experts: int):
 
 
 def _status_of(status, x) -> dict:
-    """The kernels' status word, for the grouped products that have bounded waits (they run on the GPU alone)."""
+    """The kernels' status word, for kernels that report in it on the GPU (stand-ins for them report nothing)."""
     return {"status": status} if status is not None and x.is_cuda else {}
 
 
@@ -1303,7 +1303,8 @@ def linear_scan_memory(state_row: torch.Tensor, num_heads: int, head_dim: int, v
 
 
 def linear_scan(x, state, cu_q, state_slots, *, num_heads, head_dim, v_dim, mode: str, q_off: int, k_off: int,
-                v_off: int, gate_bias=None, lower=None, decay=None, qk_group: int = 1, decay_off: int = 0) -> torch.Tensor:
+                v_off: int, gate_bias=None, lower=None, decay=None, qk_group: int = 1, decay_off: int = 0,
+                status=None) -> torch.Tensor:
     """``S_t = diag(a_t) S_(t-1) + k_t v_t^T; o_t = S_t^T q_t`` per head over the step's tokens, sequence by sequence,
     from and into ``state`` [slots, floats] float32 (:func:`linear_scan_state_floats` of them per slot).  The columns
     of ``x`` from ``q_off`` / ``k_off`` / ``v_off`` hold a product's q, gate-or-key and v.  ``mode`` ``"gated_write"``:
@@ -1312,10 +1313,12 @@ def linear_scan(x, state, cu_q, state_slots, *, num_heads, head_dim, v_dim, mode
     k, v as they stand in ``x``, which is then float32 (a kernel before has prepared them); ``"token_decay"``: the
     same with ``a = x[t, decay_off + head]``, a scalar per head and token, and ``qk_group`` heads in a row sharing one
     q and one k (the q and k columns then hold ``num_heads / qk_group`` heads).  Returns float32
-    [tokens, heads * v_dim]."""
+    [tokens, heads * v_dim].  A sequence whose rows or state slot are not there is reported in ``status`` and not
+    walked: its rows of the result are zeros."""
     out = torch.empty((x.shape[0], num_heads * v_dim), dtype=torch.float32, device=x.device)
     ext().linear_scan(x, state, cu_q, state_slots, out, num_heads, head_dim, v_dim, LINEAR_SCAN_MODES[mode], int(q_off),
-                      int(k_off), int(v_off), gate_bias, lower, decay, int(qk_group), int(decay_off))
+                      int(k_off), int(v_off), gate_bias, lower, decay, int(qk_group), int(decay_off),
+                      **_status_of(status, x))
     _launched()
     return out
 

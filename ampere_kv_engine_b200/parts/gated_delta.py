@@ -179,7 +179,7 @@ class GatedDelta(Mixer):
         qkv, coef = ops.delta_prep(x, self.conv, self.rate_log, self.step_bias, cache.state, ctx.cu_q,
                                    ctx.state_slots, unit_eps=self.unit_eps, **sizes, **more, **prep)
         return ops.delta_scan(qkv, coef, x, self.norm_weight, cache.state, ctx.cu_q, ctx.state_slots,
-                              norm_eps=self.norm_eps, **sizes, **more, **scan)
+                              norm_eps=self.norm_eps, status=ctx.status, **sizes, **more, **scan)
 
     def forward(self, x, ctx, cache):
         return ops.linear(self.heads_forward(x, ctx, cache), self.w_o, status=ctx.status)

@@ -95,7 +95,8 @@ class Hgrn2(_LinearMemory):
         x = ops.linear(x, self.w_in, status=ctx.status)
         o = ops.linear_scan(x, cache.state, ctx.cu_q, ctx.state_slots, num_heads=self.num_heads,
                             head_dim=self.head_dim, v_dim=self.v_dim, mode="gated_write", q_off=0,
-                            k_off=self.qk_width, v_off=2 * self.qk_width, gate_bias=self.gate_bias, lower=self.lower)
+                            k_off=self.qk_width, v_off=2 * self.qk_width, gate_bias=self.gate_bias, lower=self.lower,
+                            status=ctx.status)
         return ops.group_norm_gate(o, self.norm_weight, group=self.v_dim, eps=self.norm_eps, out_dtype=x.dtype,
                                    factor=self.out_scale)
 
@@ -141,7 +142,7 @@ class LightningAttention(_LinearMemory):
         x = ops.linear(x, self.w_in, status=ctx.status)
         o = ops.linear_scan(x, cache.state, ctx.cu_q, ctx.state_slots, num_heads=self.num_heads,
                             head_dim=self.head_dim, v_dim=self.v_dim, mode="constant_decay", q_off=0,
-                            k_off=self.qk_width, v_off=2 * self.qk_width, decay=self.decay)
+                            k_off=self.qk_width, v_off=2 * self.qk_width, decay=self.decay, status=ctx.status)
         return ops.group_norm_gate(o, self.norm_weight, group=self.v_width, eps=self.norm_eps, out_dtype=x.dtype,
                                    factor=self.out_scale, x=x, gate_off=2 * self.qk_width + self.v_width)
 
@@ -211,7 +212,7 @@ class Retention(_LinearMemory):
                                v_off=off + 2 * self.qk_width, k_scale=self.key_scale)
         o = ops.linear_scan(rows, cache.state, ctx.cu_q, ctx.state_slots, num_heads=self.num_heads,
                             head_dim=self.head_dim, v_dim=self.v_dim, mode="plain_decay", q_off=0,
-                            k_off=self.qk_width, v_off=2 * self.qk_width, decay=self.decay)
+                            k_off=self.qk_width, v_off=2 * self.qk_width, decay=self.decay, status=ctx.status)
         return ops.group_norm_gate(o, None, group=self.v_dim, eps=self.norm_eps, out_dtype=x.dtype,
                                    factor=self.out_scale, x=x, gate_off=off + 2 * self.qk_width + self.v_width,
                                    gate="silu")

@@ -98,7 +98,8 @@ class Mamba2(Mixer):
                             step_off=self.inner + self.channels)
         o = ops.linear_scan(rows, cache.state, ctx.cu_q, ctx.state_slots, num_heads=self.num_heads,
                             head_dim=self.state_dim, v_dim=self.v_dim, mode="token_decay", q_off=0, k_off=gn,
-                            v_off=2 * gn, qk_group=self.num_heads // self.groups, decay_off=2 * gn + self.inner)
+                            v_off=2 * gn, qk_group=self.num_heads // self.groups, decay_off=2 * gn + self.inner,
+                            status=ctx.status)
         ops.conv_tail(x, cache.state, ctx.cu_q, ctx.state_slots, tail_off=self.memory, conv_off=self.inner,
                       channels=self.channels, taps=self.taps)
         return ops.group_norm_gate(o, self.norm_weight, group=self.inner // self.norm_groups, eps=self.norm_eps,
