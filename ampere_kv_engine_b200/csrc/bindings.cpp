@@ -77,6 +77,10 @@ int* status_ptr(const OptTensor& status) {
   return status->data_ptr<int>();
 }
 
+// The bound of a kernel's waits as a caller gives it: negative for the package's own, otherwise a smaller one (0: every wait
+// gives up at once, with which the tests reach what a kernel does then).
+uint32_t wait_tries(int64_t limit) { return limit < 0 || limit > 0xffffffffLL ? 0xffffffffu : (uint32_t)limit; }
+
 void check_launch(int err, const char* what) {
   AKV_CHECK(err == 0, what, ": launch failed: ", cudaGetErrorString((cudaError_t)err));
 }
@@ -854,7 +858,7 @@ void latent_gather(const Tensor& cache, const Tensor& block_table, const Tensor&
 void latent_prompt_attention(const Tensor& q, const Tensor& q_rows, const Tensor& kv, const Tensor& latents, Tensor& out,
                              const Tensor& plan, int64_t num_seqs, int64_t num_tiles, int64_t heads, int64_t dim,
                              int64_t rot_dim, int64_t v_dim, int64_t rank, int64_t window, double scale,
-                             const OptTensor& gate, const OptTensor& sink, const OptTensor& status) {
+                             const OptTensor& gate, const OptTensor& sink, const OptTensor& status, int64_t wait_limit) {
   AKV_CHECK(q.is_cuda() && q.dim() == 2 && q.stride(1) == 1 && q.size(1) >= heads * (dim + rot_dim) &&
                 reinterpret_cast<uintptr_t>(q.data_ptr()) % 16 == 0,
             "latent_prompt_attention: q [tokens, heads * (dim + rot_dim) and more], rows contiguous, 16-byte aligned");
@@ -905,6 +909,7 @@ void latent_prompt_attention(const Tensor& q, const Tensor& q_rows, const Tensor
   p.window = (int)window;
   p.scale = (float)scale;
   p.status = status_ptr(status);
+  p.wait_limit = wait_tries(wait_limit);
   c10::cuda::CUDAGuard guard(kv.device());
   check_launch(akv::launch_latent_prompt(p, stream_of(kv)), "latent_prompt_attention");
 }
@@ -2175,7 +2180,7 @@ void moe_sort(const Tensor& chosen, Tensor& order, Tensor& offsets) {
 }
 
 void moe_gate_up(const Tensor& x, const Tensor& w, const Tensor& order, const Tensor& offsets, Tensor& act, int64_t top,
-                 double limit, double slope, int64_t form, double up_offset, const OptTensor& status) {
+                 double limit, double slope, int64_t form, double up_offset, const OptTensor& status, int64_t wait_limit) {
   check_cuda(x, "x");
   check_cuda(w, "w");
   check_cuda(act, "act");
@@ -2206,13 +2211,14 @@ void moe_gate_up(const Tensor& x, const Tensor& w, const Tensor& order, const Te
   AKV_CHECK(form >= 0 && form <= 4, "form: 0 by size, 1 float arithmetic, 2 mma.sync tiles, 3 few rows, 4 tcgen05 tiles");
   p.force_plain = (int)form;
   p.status = status_ptr(status);
+  p.wait_limit = wait_tries(wait_limit);
   c10::cuda::CUDAGuard guard(x.device());
   check_launch(akv::launch_moe_gemm(p, akv::kMoeGated, stream_of(x)), "moe_gate_up");
 }
 
 // act[r] = activation(w[expert of sorted row r] x[token of that row]): experts without a gate.
 void moe_up(const Tensor& x, const Tensor& w, const Tensor& order, const Tensor& offsets, Tensor& act, int64_t top,
-            int64_t activation, int64_t form, const OptTensor& status) {
+            int64_t activation, int64_t form, const OptTensor& status, int64_t wait_limit) {
   check_cuda(x, "x");
   check_cuda(w, "w");
   check_cuda(act, "act");
@@ -2241,12 +2247,13 @@ void moe_up(const Tensor& x, const Tensor& w, const Tensor& order, const Tensor&
   p.dtype = dtype_code(x, "x");
   p.force_plain = (int)form;
   p.status = status_ptr(status);
+  p.wait_limit = wait_tries(wait_limit);
   c10::cuda::CUDAGuard guard(x.device());
   check_launch(akv::launch_moe_gemm(p, akv::kMoeUp, stream_of(x)), "moe_up");
 }
 
 void moe_down(const Tensor& act, const Tensor& w, const Tensor& order, const Tensor& offsets, const Tensor& weights,
-              Tensor& out, int64_t form, const OptTensor& status) {
+              Tensor& out, int64_t form, const OptTensor& status, int64_t wait_limit) {
   check_cuda(act, "act");
   check_cuda(w, "w");
   check_same(act, w, "act", "w");
@@ -2273,6 +2280,7 @@ void moe_down(const Tensor& act, const Tensor& w, const Tensor& order, const Ten
   AKV_CHECK(form >= 0 && form <= 4, "form: 0 by size, 1 float arithmetic, 2 mma.sync tiles, 3 few rows, 4 tcgen05 tiles");
   p.force_plain = (int)form;
   p.status = status_ptr(status);
+  p.wait_limit = wait_tries(wait_limit);
   c10::cuda::CUDAGuard guard(act.device());
   check_launch(akv::launch_moe_gemm(p, akv::kMoeDown, stream_of(act)), "moe_down");
 }
@@ -2489,7 +2497,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("latent_prompt_attention", &latent_prompt_attention, py::arg("q"), py::arg("q_rows"), py::arg("kv"),
         py::arg("latents"), py::arg("out"), py::arg("plan"), py::arg("num_seqs"), py::arg("num_tiles"), py::arg("heads"),
         py::arg("dim"), py::arg("rot_dim"), py::arg("v_dim"), py::arg("rank"), py::arg("window"), py::arg("scale"),
-        py::arg("gate") = py::none(), py::arg("sink") = py::none(), py::arg("status") = py::none());
+        py::arg("gate") = py::none(), py::arg("sink") = py::none(), py::arg("status") = py::none(),
+        py::arg("wait_limit") = -1);
   m.def("moe_route", &moe_route, py::arg("logits"), py::arg("correction"), py::arg("chosen"), py::arg("weights"),
         py::arg("groups"), py::arg("keep_groups"), py::arg("group_top"), py::arg("scale"), py::arg("weight_eps"),
         py::arg("score_kind") = 0, py::arg("normalize") = true, py::arg("bias") = py::none());
@@ -2497,11 +2506,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("moe_sort", &moe_sort, py::arg("chosen"), py::arg("order"), py::arg("offsets"));
   m.def("moe_gate_up", &moe_gate_up, py::arg("x"), py::arg("w"), py::arg("order"), py::arg("offsets"), py::arg("act"),
         py::arg("top"), py::arg("limit"), py::arg("slope"), py::arg("form") = 0, py::arg("up_offset") = 1.0,
-        py::arg("status") = py::none());
+        py::arg("status") = py::none(), py::arg("wait_limit") = -1);
   m.def("moe_up", &moe_up, py::arg("x"), py::arg("w"), py::arg("order"), py::arg("offsets"), py::arg("act"),
-        py::arg("top"), py::arg("activation"), py::arg("form") = 0, py::arg("status") = py::none());
+        py::arg("top"), py::arg("activation"), py::arg("form") = 0, py::arg("status") = py::none(), py::arg("wait_limit") = -1);
   m.def("moe_down", &moe_down, py::arg("act"), py::arg("w"), py::arg("order"), py::arg("offsets"), py::arg("weights"),
-        py::arg("out"), py::arg("form") = 0, py::arg("status") = py::none());
+        py::arg("out"), py::arg("form") = 0, py::arg("status") = py::none(), py::arg("wait_limit") = -1);
   m.def("moe_combine", &moe_combine, py::arg("parts"), py::arg("shared"), py::arg("out"), py::arg("top"),
         py::arg("chosen") = py::none(), py::arg("pair_weights") = py::none(), py::arg("x") = py::none(),
         py::arg("first_identity") = 0);

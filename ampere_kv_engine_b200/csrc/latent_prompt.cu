@@ -23,7 +23,8 @@
 // before: 2,048 tokens, 32 heads of 128 + 64, rank 512: behind a window of 1,024 7.35 -> 3.44 ms, over all keys 5.39 ->
 // 2.75 ms, after 2,048 earlier tokens 10.11 -> 2.93 ms.
 //
-// Every wait is bounded; a wait that runs out sets kWaitTimeout and the CTA frees its TMEM and leaves.
+// Every wait is bounded; when one runs out, the CTA sets kWaitTimeout, waits (again with a bound) for its copies and
+// MMAs under way, frees its TMEM and leaves.
 #include "common.cuh"
 #include "launchers.h"
 #include "tcgen05.cuh"
@@ -48,7 +49,9 @@ struct Shared {
   uint64_t s_ready[2];       // scores of a block are in TMEM buffer (block & 1)
   uint64_t p_ready[2];       // P of a block is in tensor memory: 256 arrivals
   uint64_t pv_done[2];       // O holds the sum through block j: barrier (j & 1), phase (j >> 1)
+  uint64_t drained[2];       // after a wait that ran out: the MMAs of each issuing warp
   uint32_t tmem;
+  int failed;
   float exchange[2][2][kRows];      // [block parity][half][row]: maxima, at the end sums
 };
 constexpr int kSmemBytes = 1024 + kQBytes + kStages * kStageBytes + (int)sizeof(Shared);
@@ -206,7 +209,9 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
       tc::mbar_init(&s.s_ready[i], 1);
       tc::mbar_init(&s.p_ready[i], kSoftmax);
       tc::mbar_init(&s.pv_done[i], 1);
+      tc::mbar_init(&s.drained[i], 1);
     }
+    s.failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kScoreWarp) tc::tmem_alloc(&s.tmem, kTmemColumns);
@@ -216,6 +221,9 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
   const uint32_t tmem = s.tmem;
   pdl_wait();
   bool ok = true;
+  int keys = 0, values = 0;      // blocks whose copies have been issued (the copying thread's)
+  const uint32_t tries = min(p.wait_limit, kWaitLimit);
+  auto wait = [&](uint64_t* bar, uint32_t parity) -> bool { return tc::mbar_wait(bar, parity, tries); };
 
   if (warp == kCopyWarp) {
     if (lane == 0) {
@@ -225,8 +233,9 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
       tma_load_3d(q_smem + 2 * kChunk, &q_rot_map, p.rank, head, q0, &s.q_full);
       auto fetch_keys = [&](int b) -> bool {
         const int st = b % kStages, row = base + lo_row + b * kKeys;
-        if (b >= kStages && !tc::mbar_wait(&s.k_empty[st], ((b / kStages) - 1) & 1)) return false;
+        if (b >= kStages && !wait(&s.k_empty[st], ((b / kStages) - 1) & 1)) return false;
         uint8_t* dst = kv_smem + st * kStageBytes;
+        keys = b + 1;
         tc::mbar_expect_tx(&s.k_full[st], kKBytes);
         tma_load_3d(dst, &k_map, 0, head, row, &s.k_full[st]);
         tma_load_3d(dst + kChunk, &k_map, 64, head, row, &s.k_full[st]);
@@ -235,8 +244,9 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
       };
       auto fetch_values = [&](int b) -> bool {
         const int st = b % kStages, row = base + lo_row + b * kKeys;
-        if (b >= kStages && !tc::mbar_wait(&s.v_empty[st], ((b / kStages) - 1) & 1)) return false;
+        if (b >= kStages && !wait(&s.v_empty[st], ((b / kStages) - 1) & 1)) return false;
         uint8_t* dst = kv_smem + st * kStageBytes + kKBytes;
+        values = b + 1;
         tc::mbar_expect_tx(&s.v_full[st], kVBytes);
         tma_load_3d(dst, &v_map, 0, head, row, &s.v_full[st]);
         tma_load_3d(dst + kChunk, &v_map, 64, head, row, &s.v_full[st]);
@@ -253,12 +263,12 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
     if (lane == 0) {
       constexpr uint32_t id_s = tc::umma_idesc(kKeys);
       const uint32_t q_addr = tc::smem_u32(q_smem);
-      if (!tc::mbar_wait(&s.q_full, 0)) ok = false;
+      if (!wait(&s.q_full, 0)) ok = false;
       for (int b = 0; b < num_blocks && ok; ++b) {
         const int st = b % kStages;
         // the scores of block b go into buffer b & 1, where P of block b - 2 lay: P V of that block must be done
-        if (b >= 2 && !tc::mbar_wait(&s.pv_done[b & 1], ((b - 2) >> 1) & 1)) { ok = false; break; }
-        if (!tc::mbar_wait(&s.k_full[st], (b / kStages) & 1)) { ok = false; break; }
+        if (b >= 2 && !wait(&s.pv_done[b & 1], ((b - 2) >> 1) & 1)) { ok = false; break; }
+        if (!wait(&s.k_full[st], (b / kStages) & 1)) { ok = false; break; }
         tc::fence_after();
         const uint32_t k_addr = tc::smem_u32(kv_smem + st * kStageBytes);
 #pragma unroll
@@ -275,8 +285,8 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
       constexpr uint32_t id_o = tc::umma_idesc(128) | (1u << 16);         // B MN-major
       for (int b = 0; b < num_blocks && ok; ++b) {
         const int st = b % kStages;
-        if (!tc::mbar_wait(&s.p_ready[b & 1], (b >> 1) & 1)) { ok = false; break; }
-        if (!tc::mbar_wait(&s.v_full[st], (b / kStages) & 1)) { ok = false; break; }
+        if (!wait(&s.p_ready[b & 1], (b >> 1) & 1)) { ok = false; break; }
+        if (!wait(&s.v_full[st], (b / kStages) & 1)) { ok = false; break; }
         tc::fence_after();
         const uint32_t v_addr = tc::smem_u32(kv_smem + st * kStageBytes + kKBytes);
         const uint32_t p_tmem = tmem + (b & 1) * kKeys;
@@ -288,7 +298,8 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
       }
     }
   } else {
-    // softmax: two threads per query row, warps w and w + 4 share the TMEM lanes 32 (w % 4) .. + 31
+    // softmax: two threads per query row, warps w and w + 4 share the TMEM lanes 32 (w % 4) .. + 31; a warp agrees on
+    // every wait's outcome, since its accesses of tensor memory are the whole warp's
     const int half = warp >> 2, row = (warp & 3) * 32 + lane, pair_bar = 1 + (warp & 3);
     const bool live = row < nq;
     const int pos = tile_pos + row;
@@ -303,7 +314,7 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
     }
     for (int b = 0; b < num_blocks; ++b) {
       const int key0 = key_begin + b * kKeys + half * 64;      // this thread's first key of the block
-      if (ok && !tc::mbar_wait(&s.s_ready[b & 1], (b >> 1) & 1)) ok = false;
+      ok = __all_sync(0xffffffffu, ok && wait(&s.s_ready[b & 1], (b >> 1) & 1));
       tc::fence_after();
       uint32_t raw[2][32];
       if (ok) {
@@ -337,7 +348,7 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
       if (__any_sync(0xffffffffu, raise)) {
         const float alpha = (raise && m_ref != -CUDART_INF_F) ? ex2(m_ref - bmax) : 1.f;
         if (b > 0) {
-          if (ok && !tc::mbar_wait(&s.pv_done[(b - 1) & 1], ((b - 1) >> 1) & 1)) ok = false;
+          ok = __all_sync(0xffffffffu, ok && wait(&s.pv_done[(b - 1) & 1], ((b - 1) >> 1) & 1));
           tc::fence_after();
           if (ok) {
 #pragma unroll 1
@@ -382,7 +393,7 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
     pair_sync(pair_bar);
     l = sums[0][row] + sums[1][row];
     // the products run in order, so the last one done means all are
-    if (num_blocks > 0 && ok && !tc::mbar_wait(&s.pv_done[(num_blocks - 1) & 1], ((num_blocks - 1) >> 1) & 1)) ok = false;
+    if (num_blocks > 0) ok = __all_sync(0xffffffffu, ok && wait(&s.pv_done[(num_blocks - 1) & 1], ((num_blocks - 1) >> 1) & 1));
     tc::fence_after();
     float inv = (ok && l > 0.f) ? 1.f / l : 0.f;
     if (p.gate != nullptr && live) inv *= p.gate[(int64_t)(q0 + row) * p.heads + head];
@@ -410,9 +421,25 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
       }
     }
   }
-  if (!ok && lane == 0) set_status(p.status, kWaitTimeout);
+  if (!ok && lane == 0) {
+    set_status(p.status, kWaitTimeout);
+    s.failed = 1;
+  }
   tc::fence_before();
   __syncthreads();
+  if (s.failed) {
+    // what is under way and nobody waits for any more: it lands before the shared and the tensor memory go
+    if (warp == kCopyWarp && lane == 0) {
+      tc::mbar_wait(&s.q_full, 0);
+      for (int b = max(0, keys - kStages); b < keys; ++b) tc::mbar_wait(&s.k_full[b % kStages], (b / kStages) & 1);
+      for (int b = max(0, values - kStages); b < values; ++b) tc::mbar_wait(&s.v_full[b % kStages], (b / kStages) & 1);
+    }
+    if ((warp == kScoreWarp || warp == kPvWarp) && lane == 0) {
+      tc::umma_commit(&s.drained[warp - kScoreWarp]);
+      tc::mbar_wait(&s.drained[warp - kScoreWarp], 0);
+    }
+    __syncthreads();
+  }
   if (warp == kScoreWarp) tc::tmem_free(tmem, kTmemColumns);
 }
 

@@ -284,6 +284,7 @@ struct LatentPromptParams {
   int num_seqs, num_tiles, heads, dim, rot_dim, v_dim, rank, window;
   float scale;
   int* status;
+  uint32_t wait_limit;         // most tries of a wait, if fewer than the package's bound
 };
 bool latent_prompt_supported(int dim, int rot_dim, int v_dim, int rank);
 int launch_latent_prompt(const LatentPromptParams& p, cudaStream_t stream);
@@ -460,6 +461,7 @@ struct MoeGemmParams {
                                // 4: tcgen05 tiles (routed_experts_tc.cu)
   int activation;              // up: an Activation
   int* status;                 // kernels' status word, or null
+  uint32_t wait_limit;         // most tries of a wait in the tcgen05 form, if fewer than the package's bound
 };
 // most (token, choice) pairs that the few-rows form takes by itself: first products of hidden sizes below the tcgen05
 // form's K block (against mma.sync tiles at 8 tokens, 64 experts of 1,024 x 4,096: 103 against 111 us; the down product

@@ -23,8 +23,8 @@
 // what keeps a prompt from it is the ring: at 200 rows a stage is 57 KB, three fit, and the memory's latency is not
 // covered (DRAM at 39 %, the tensor pipe and the crossbar far below their limits).
 //
-// Every wait is bounded; a wait that runs out sets kWaitTimeout in the status word, copies under way are waited for,
-// and the CTA frees its TMEM and leaves.
+// Every wait is bounded; a wait that runs out sets kWaitTimeout in the status word, copies and MMAs under way are waited
+// for, and the CTA frees its TMEM and leaves.
 #include "common.cuh"
 #include "launchers.h"
 #include "tcgen05.cuh"
@@ -46,6 +46,7 @@ constexpr int kThreads = 32 * (2 + kRowWarps + kEpilogueWarps);
 
 struct Shared {
   uint64_t full[kMaxStages], empty[kMaxStages], acc_full, acc_empty;
+  uint64_t drained;                           // after a wait that ran out: the MMAs under way
   uint32_t tmem;
   int widest;                                 // rows of the widest tile
   int failed;
@@ -106,6 +107,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, MoeGemmParams p) {
     }
     tc::mbar_init(&s.acc_full, 1);
     tc::mbar_init(&s.acc_empty, kEpilogueWarps);
+    tc::mbar_init(&s.drained, 1);
     s.failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -145,6 +147,8 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, MoeGemmParams p) {
   const int stages = min(kMaxStages, kRing / stage_bytes);
   const int blocks = (p.k + kK - 1) / kK;
   bool ok = true;
+  const uint32_t tries = min(p.wait_limit, kWaitLimit);
+  auto wait = [&](uint64_t* bar, uint32_t parity) -> bool { return tc::mbar_wait(bar, parity, tries); };
   int stage = 0, issued = 0;
   uint32_t phase = 0;
 
@@ -154,7 +158,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, MoeGemmParams p) {
         const Tile t = tile_of(s, p.offsets, p.experts, m_tiles, tile);
         const int w_row = t.expert * (GATED ? 2 : 1) * p.n + t.m * kFeatures;
         for (int kb = 0; kb < blocks; ++kb) {
-          if (!tc::mbar_wait(&s.empty[stage], phase ^ 1)) {
+          if (!wait(&s.empty[stage], phase ^ 1)) {
             ok = false;
             break;
           }
@@ -198,7 +202,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, MoeGemmParams p) {
         source[i] = 16 * i < t.rows ? (FIRST ? p.order[r] / p.top : r) : 0;
       }
       for (int kb = 0; kb < blocks; ++kb) {
-        ok = __all_sync(0xffffffffu, tc::mbar_wait(&s.empty[stage], phase ^ 1));
+        ok = __all_sync(0xffffffffu, wait(&s.empty[stage], phase ^ 1));
         if (!ok) break;
         const int k = kb * kK + piece * 8;
         const bool inside = k < p.k;
@@ -228,13 +232,13 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, MoeGemmParams p) {
       int done = 0;
       for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++done) {
         const uint32_t idesc = tc::umma_idesc(round16(tile_of(s, p.offsets, p.experts, m_tiles, tile).rows));
-        if (done > 0 && !tc::mbar_wait(&s.acc_empty, (uint32_t)(done - 1) & 1u)) {
+        if (done > 0 && !wait(&s.acc_empty, (uint32_t)(done - 1) & 1u)) {
           ok = false;
           break;
         }
         tc::fence_after();
         for (int kb = 0; kb < blocks; ++kb) {
-          if (!tc::mbar_wait(&s.full[stage], phase)) {
+          if (!wait(&s.full[stage], phase)) {
             ok = false;
             break;
           }
@@ -265,7 +269,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, MoeGemmParams p) {
     for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++done) {
       const Tile t = tile_of(s, p.offsets, p.experts, m_tiles, tile);
       const int feature = t.m * kFeatures + quarter * 32 + lane;
-      ok = __all_sync(0xffffffffu, tc::mbar_wait(&s.acc_full, (uint32_t)done & 1u));
+      ok = __all_sync(0xffffffffu, wait(&s.acc_full, (uint32_t)done & 1u));
       if (!ok) break;
       tc::fence_after();
 #pragma unroll 1
@@ -316,9 +320,16 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, MoeGemmParams p) {
   }
   tc::fence_before();
   __syncthreads();
-  if (s.failed && threadIdx.x == 0) {
-    // weights under way that nobody waits for any more: time to land before the shared memory goes
-    for (int i = max(0, issued - stages); i < issued; ++i) tc::mbar_wait(&s.full[i % stages], (uint32_t)(i / stages) & 1u);
+  if (s.failed) {
+    // what is under way and nobody waits for any more: it lands before the shared and the tensor memory go (a stage whose
+    // rows were never announced does not fill; its weights have long landed when the wait for it gives up)
+    if (threadIdx.x == 0)
+      for (int i = max(0, issued - stages); i < issued; ++i) tc::mbar_wait(&s.full[i % stages], (uint32_t)(i / stages) & 1u);
+    if (warp == 1 && lane == 0) {
+      tc::umma_commit(&s.drained);
+      tc::mbar_wait(&s.drained, 0);
+    }
+    __syncthreads();
   }
   if (warp == 1) tc::tmem_free(tmem, 512);
 }
