@@ -370,21 +370,25 @@ latent_prompt_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_con
       }
       // a row that has seen no key yet subtracts 0, so that 2^(-inf - 0) = 0 and not 2^(-inf + inf)
       const float m_sub = m_ref == -CUDART_INF_F ? 0.f : m_ref;
+      // The row's sum takes the weights as P V takes them, rounded to bfloat16: the reference lies up to 2^8 below the
+      // maximum, so the largest weight is no power of two, and its rounding would stay in the result of a row that one key
+      // dominates; taken on both sides it cancels.
       uint32_t packed[32];
-      float part[4] = {0.f, 0.f, 0.f, 0.f};
+      float2 part[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
       for (int j = 0; j < 64; j += 2) {
         const float pa = ex2(fmaf(__uint_as_float(raw[j >> 5][j & 31]), scale_log2, -m_sub));
         const float pb = ex2(fmaf(__uint_as_float(raw[(j + 1) >> 5][(j + 1) & 31]), scale_log2, -m_sub));
-        part[(j >> 1) & 3] += pa + pb;
         __nv_bfloat162 h = __floats2bfloat162_rn(pa, pb);
-        packed[j >> 1] = *reinterpret_cast<uint32_t*>(&h);
+        const uint32_t both = *reinterpret_cast<uint32_t*>(&h);
+        packed[j >> 1] = both;
+        part[(j >> 1) & 1] = add2(part[(j >> 1) & 1], make_float2(__uint_as_float(both << 16), __uint_as_float(both & 0xffff0000u)));
       }
       if (ok) {
         tmem_store32(lane_base + (b & 1) * kKeys + half * 32, packed);
         tmem_wait_store();
       }
-      l += (part[0] + part[1]) + (part[2] + part[3]);
+      l += (part[0].x + part[0].y) + (part[1].x + part[1].y);
       tc::fence_before();
       tc::mbar_arrive(&s.p_ready[b & 1]);
     }

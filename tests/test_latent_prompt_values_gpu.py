@@ -25,3 +25,20 @@ def test_a_latent_that_is_not_finite(value, window, key, column):
     assert bool(((first - want).abs() <= bound)[~sees].all())
     want, bound = case.plain(1)
     assert bool(((got[120:] - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("window,sink,sharpness", [(1, -4.0, 1.0), (2, -4.0, 1.0), (1, -12.0, 1.0), (0, None, 12.0)])
+def test_a_row_that_one_key_dominates(window, sink, sharpness):
+    """Such a row is nearly that key's value: a weight's rounding must not stay in it, only the result's.  (With a sink the
+    walk refers its weights to the sink's score while no key stands far above it, so the largest is no power of two.)"""
+    from ampere_kv_engine_b200.kernels import ops
+
+    heads = 6
+    case = LatentCase([300], [900], heads=heads, window=window, seed=5,
+                      sink=None if sink is None else torch.full((heads,), sink, device="cuda"))
+    case.scale *= sharpness
+    got, (want, _) = case.run(ops), case.plain(0)
+    # rounding the exact result alone; what the sink's share leaves of a weight's rounding, and further keys', fits into a
+    # quarter of it (a weight's whole rounding would make it 1.4 times as much)
+    rounding = (want.bfloat16().double() - want).norm()
+    assert float((got - want).norm()) <= 1.25 * float(rounding)
