@@ -497,7 +497,7 @@ def rotate_pairs(x, out, positions, inv_freq, *, heads, cols, rotary_dims, in_of
 
 
 LATENT_TILE = 128          # query tokens of a tile, keys of a block: a sequence's gathered rows are a multiple of it
-#: most bytes of keys and values that a step writes out; a step over longer contexts stays in the latent space
+#: most bytes of keys and values that are written out at a time; a portion that needs more stays in the latent space
 LATENT_PLAN_BYTES = 1 << 30
 
 
@@ -515,16 +515,22 @@ class LatentPlan:
         return self
 
 
-def latent_plan(q_lens: list[int], ctx_lens: list[int], window: int) -> LatentPlan | None:
-    """The plan of the sequences with more than one new token (None without any): host lengths in, tiles with the most
-    keys first."""
+def _latent_rows(n: int, c: int, window: int) -> tuple[int, int]:
+    """The first key that a portion of n tokens at the end of c sees, and the rows that are gathered for it."""
+    first = max(0, c - n - window + 1) if window else 0
+    return first, (c - first + LATENT_TILE - 1) // LATENT_TILE * LATENT_TILE
+
+
+def latent_plan(q_lens: list[int], ctx_lens: list[int], window: int, only: set[int] | None = None) -> LatentPlan | None:
+    """The plan of the sequences with more than one new token (of those in ``only``, if given; None without any): host
+    lengths in, tiles with the most keys first."""
     numbers, tiles, rows, row0, tokens, pairs = [], [], 0, 0, 0, 0
     for s, (n, c) in enumerate(zip(q_lens, ctx_lens)):
-        if n > 1:
-            first = max(0, c - n - window + 1) if window else 0
+        if n > 1 and (only is None or s in only):
+            first, gathered = _latent_rows(n, c, window)
             index = len(numbers) // 6
             numbers += [rows, first, c, n, row0, s]
-            rows += (c - first + LATENT_TILE - 1) // LATENT_TILE * LATENT_TILE
+            rows += gathered
             tokens += n
             pairs += n * (c - first)
             for t in range(0, n, LATENT_TILE):
@@ -538,6 +544,55 @@ def latent_plan(q_lens: list[int], ctx_lens: list[int], window: int) -> LatentPl
     for _, index, t in tiles:
         numbers += [index, t]
     return LatentPlan(numbers, count, len(tiles), rows, tokens, pairs)
+
+
+class LatentStep:
+    """How a step's tokens go through latents: ``plans``, the portions whose keys and values are written out, in groups
+    one after the other; all other sequences stay in the latent space: the single tokens (which have tiles of their own
+    in the step) and the portions that ``tiles`` lists (sequence, first batch row, rows).  ``rows``: the batch rows up
+    to the last one that stays."""
+
+    def __init__(self, plans: list[LatentPlan], tiles: list[tuple[int, int, int]], rows: int):
+        self.plans, self.rows, self.num_tiles = plans, rows, len(tiles)
+        self.numbers = [v for plan in plans for v in plan.numbers] + [t[i] for i in range(3) for t in tiles]
+        self.tiles = None
+
+    def to(self, device):
+        return self.place(torch.tensor(self.numbers, dtype=torch.int32).pin_memory().to(device, non_blocking=True))
+
+    def place(self, numbers: torch.Tensor):
+        """``numbers``: this object's numbers on the device."""
+        at = 0
+        for plan in self.plans:
+            plan.plan = numbers[at:at + len(plan.numbers)]
+            at += len(plan.numbers)
+        self.tiles = tuple(numbers[at + i * self.num_tiles:at + (i + 1) * self.num_tiles] for i in range(3))
+        return self
+
+
+def latent_step(q_lens: list[int], ctx_lens: list[int], *, window: int, portion: int, row_bytes: int, q_tile: int,
+                group_bytes: int, most_bytes: int) -> LatentStep | None:
+    """The step's :class:`LatentStep`, or None when nothing is written out.  A portion is written out when it has at least
+    ``portion`` new tokens and its own gathered rows, of ``row_bytes`` of keys and values each, take at most
+    ``most_bytes``: what becomes of it does not depend on what else the step holds.  A group takes ``group_bytes`` or is
+    one portion."""
+    groups, tiles, kept, size, row0 = [], [], 0, 0, 0
+    for s, (n, c) in enumerate(zip(q_lens, ctx_lens)):
+        own = _latent_rows(n, c, window)[1] * row_bytes
+        if n > 1 and n >= portion and own <= most_bytes:
+            if not groups or size + own > group_bytes:
+                groups.append(set())
+                size = 0
+            groups[-1].add(s)
+            size += own
+        else:
+            if n > 1:
+                tiles += [(s, row0 + q0, min(q_tile, n - q0)) for q0 in range(0, n, q_tile)]
+            kept = row0 + n
+        row0 += n
+    if not groups:
+        return None
+    return LatentStep([latent_plan(q_lens, ctx_lens, window, only) for only in groups], tiles, kept)
 
 
 def latent_prompt_takes(dtype: torch.dtype, device, dim: int, rot_dim: int, v_dim: int, rank: int) -> bool:

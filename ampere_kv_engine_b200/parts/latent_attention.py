@@ -18,7 +18,7 @@ keys and values written out: since ``q_unrot . (W_uk c) = (W_uk^T q_unrot) . c``
 space (one batched product per step) and attention runs over the rows as they are stored, every head reading the same
 row as its key and the row's first ``kv_rank`` elements as its value; the result per head is a mix of latents (times
 the head's gate), which ``W_uv`` turns into the head's output (one more batched product).  Prompt portions in bfloat16
-(:meth:`LatentAttention.prompt_plan`) share their keys among enough queries to have them written out for the step: one
+(:meth:`LatentAttention.written_out`) share their keys among enough queries to have them written out for the step: one
 product makes every head's keys and values of the rows they see, and attention runs over those (``ops.latent_prompt_attention``).  Between the first product
 and the attention stands one row-wise kernel (``ops.latent_prep``; with a query latent also ``ops.rotate_pairs`` behind
 the second product).
@@ -37,10 +37,14 @@ from .scored_attention import run_attention
 ROW_MULTIPLE = 8
 
 
-#: New tokens a portion must have, weighted by the keys it sees, for keys and values to be written out.  Measured as
-#: whole steps of four layers (us, written out against in the latent space; 32 heads of 128 + 64, rank 512, two of the
-#: layers over all keys): 16 tokens after none 827 / 870, after 2,048 913 / 994; 64 tokens 865 / 917, 965 / 1,091; 512
-#: tokens 1,112 / 1,355, 1,205 / 2,732.  At 8 tokens the two are within what such steps differ by.
+#: New tokens that a portion must have for its keys and values to be written out.  Both forms cost a key about the same
+#: number of operations per new token behind the first few, so the line does not move with the context; and it is drawn
+#: for each portion by itself, so that a request's numbers do not depend on who shares its step.  Measured as whole steps
+#: of four layers (us, written out against in the latent space; 32 heads of 128 + 64, rank 512, two of the layers over all
+#: keys): eight portions after 2,048 tokens each 1,506 / 1,444 at 8 new tokens, 1,539 / 1,497 at 16, 1,565 / 1,927 at 24,
+#: 1,752 / 2,764 at 64; eight from the start 1,069 / 1,133 at 16; one portion after 2,048 tokens 955 / 1,032 at 16.  Below
+#: 16 tokens a written-out key is hardly shared: eight portions of 2 tokens after 2,048 take 1,448 / 1,362, and the gap
+#: grows with the context.
 LATENT_PORTION = 16
 
 
@@ -160,21 +164,20 @@ class LatentAttention(Mixer):
             # per head its key rows and its value rows: one product writes both out for a prompt
             self.w_kv = torch.cat((self.w_uk, tensors[n["uv"]].view(H, self.v_dim, self.kv_rank)), dim=1).flatten(0, 1)
 
-    def prompt_plan(self, ctx):
-        """The step's ``ops.LatentPlan`` if its prompt portions are better off with keys and values written out, else
-        None.  A key costs a portion 2 rank (dim + v_dim) operations a head once, and each (query, key) pair then 2 (dim
-        + rot_dim + v_dim) instead of 2 (2 rank + rot_dim), on a faster kernel."""
+    def written_out(self, ctx):
+        """The step's ``ops.LatentStep`` if it has prompt portions that are better off with keys and values written out,
+        else None.  A key costs a portion 2 rank (dim + v_dim) operations a head once, and each (query, key) pair then 2
+        (dim + rot_dim + v_dim) instead of 2 (2 rank + rot_dim), on a faster kernel."""
         if self.w_kv is None or not any(n > 1 for n in ctx.q_lens_host):
             return None
-        key = ("latent_prompt", self.window)
+        row_bytes = self.num_heads * (self.head_dim + self.v_dim) * 2
+        key = ("latent_prompt", self.window, row_bytes)
         if key not in ctx.shared:
-            plan = ops.latent_plan(ctx.q_lens_host, ctx.ctx_lens_host, self.window)
-            worth = plan is not None and plan.pairs >= LATENT_PORTION * plan.rows
-            ctx.shared[key] = plan.to(self.device) if worth else None
-        plan = ctx.shared[key]
-        if plan is None or plan.rows * self.num_heads * (self.head_dim + self.v_dim) * 2 > ops.LATENT_PLAN_BYTES:
-            return None
-        return plan
+            step = ops.latent_step(ctx.q_lens_host, ctx.ctx_lens_host, window=self.window, portion=LATENT_PORTION,
+                                   row_bytes=row_bytes, q_tile=ctx.q_tile, group_bytes=ops.LATENT_PLAN_BYTES,
+                                   most_bytes=ops.LATENT_PLAN_BYTES)
+            ctx.shared[key] = None if step is None else step.to(self.device)
+        return ctx.shared[key]
 
     def forward(self, x, ctx, cache, residual=None):
         if cache.writes != self.own_kv:
@@ -198,22 +201,20 @@ class LatentAttention(Mixer):
                                  in_offset=D, out_offset=rank, factor=self.rotary_factor)
         else:
             q = x[:, :self.q_width]
-        plan = self.prompt_plan(ctx)
+        step = self.written_out(ctx)
         out = torch.empty((tokens, H * self.v_dim), dtype=q.dtype, device=q.device)
-        single = getattr(ctx, "num_decode_tiles", 0)
-        if plan is None or single:
-            # in the latent space; where the prompt portions go the other way only the single tokens' rows matter, and
-            # where those come first only they are computed
-            count = single if plan is not None and all(n == 1 for n in ctx.q_lens_host[:single]) else tokens
+        if step is None or step.rows:
+            # in the latent space; where other portions go the other way, the batch rows up to the last one that stays
+            count = tokens if step is None else step.rows
             # the unrotated part of every head's query, carried into the latent space: [H, count, D] x [H, D, rank]
             torch.bmm(q[:count].unflatten(1, (H, D + R))[:, :, :D].transpose(0, 1), self.w_uk,
                       out=q_row.view(tokens, H, self.row)[:count, :, :rank].transpose(0, 1))
             mixed = torch.empty((tokens, H * rank), dtype=q.dtype, device=q.device)
             run_attention(ctx, group, q_row, rows, rows, mixed, num_heads=H, num_kv_heads=1, v_dim=rank, scale=self.scale,
-                          window=self.window, gate=gate, sink=self.sink, single_only=plan is not None)
+                          window=self.window, gate=gate, sink=self.sink, prompt_tiles=None if step is None else step.tiles)
             torch.bmm(mixed.view(tokens, H, rank)[:count].transpose(0, 1), self.w_uv,
                       out=out.view(tokens, H, self.v_dim)[:count].transpose(0, 1))              # [H, count, v_dim]
-        if plan is not None:
+        for plan in step.plans if step is not None else ():
             ops.latent_prompt_attention(q, q_row, rows, group.block_table, plan, self.w_kv, out, heads=H, dim=D, rot_dim=R,
                                         v_dim=self.v_dim, rank=rank, scale=self.scale, window=self.window, gate=gate,
                                         sink=self.sink, status=ctx.status)

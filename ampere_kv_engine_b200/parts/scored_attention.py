@@ -162,16 +162,21 @@ class ScoredAttention(Mixer):
 
 def run_attention(ctx, group, q, k_cache, v_cache, out, *, num_heads, num_kv_heads, v_dim, scale, window=0, chunk=0,
                   softcap=0.0, slopes=None, gate=None, plain=False, keep_first=0, sigmoid_weights=False, head_bias=None,
-                  out_scale=1.0, sink=None, single_only=False) -> None:
-    """``ops.scored_attention`` over the step's tiles (``single_only``: the single-token ones of a mixed step alone): the single-token tiles of a mixed step (they come first) apart
-    from the prompt tiles, each with the number of key splits that fills the GPU.  ``plain``: nothing is done to the
+                  out_scale=1.0, sink=None, prompt_tiles=None) -> None:
+    """``ops.scored_attention`` over the step's tiles: the single-token tiles of a mixed step (they come first) apart
+    from the prompt tiles, each with the number of key splits that fills the GPU.  ``prompt_tiles`` (sequences, first
+    batch rows, rows): these prompt tiles in place of the step's.  ``plain``: nothing is done to the
     scores and the plain kernels take the sizes: ``ops.paged_attention`` runs instead."""
     group_size = num_heads // num_kv_heads
     plain_tc = plain and ops.attention_takes_tensor_cores(q.dtype, q.shape[1] // num_heads, group_size,
                                                           k_cache.shape[2])
     first = getattr(ctx, "num_decode_tiles", 0)
-    for lo, hi, q_tile in ((0, first, 1), (first, ctx.num_tiles, ctx.q_tile)):
-        if hi <= lo or (single_only and lo == first):
+    all_tiles = (ctx.tile_seq, ctx.tile_q0, ctx.tile_nq)
+    if prompt_tiles is None:
+        prompt_tiles = tuple(t[first:ctx.num_tiles] for t in all_tiles)
+    for tiles, q_tile in ((tuple(t[:first] for t in all_tiles), 1), (prompt_tiles, ctx.q_tile)):
+        num_tiles = tiles[0].shape[0]
+        if num_tiles == 0:
             continue
         longest, mean = ctx.decode_contexts if q_tile == 1 else (ctx.max_context, ctx.max_context)
         for limit in (window + keep_first if window else 0, chunk):
@@ -179,10 +184,10 @@ def run_attention(ctx, group, q, k_cache, v_cache, out, *, num_heads, num_kv_hea
                 longest, mean = min(longest, limit), min(mean, limit)
         if plain:
             splits = 1 if q_tile > 1 and plain_tc else ops.choose_splits(
-                hi - lo, num_kv_heads, q_tile * group_size, longest, plain_tc, mean_context=mean)
+                num_tiles, num_kv_heads, q_tile * group_size, longest, plain_tc, mean_context=mean)
             ops.paged_attention(
-                q, k_cache, v_cache, group.block_table, ctx.cu_q, ctx.ctx_lens, ctx.tile_seq[lo:hi], ctx.tile_q0[lo:hi],
-                ctx.tile_nq[lo:hi], num_tiles=hi - lo, q_tile=q_tile, num_splits=splits, num_heads=num_heads,
+                q, k_cache, v_cache, group.block_table, ctx.cu_q, ctx.ctx_lens, *tiles,
+                num_tiles=num_tiles, q_tile=q_tile, num_splits=splits, num_heads=num_heads,
                 num_kv_heads=num_kv_heads, window=window, scale=scale, status=ctx.status, out=out)
             continue
         # kept first keys, sigmoid weights and an output factor: the tensor-core kernels take them where keys and
@@ -192,15 +197,15 @@ def run_attention(ctx, group, q, k_cache, v_cache, out, *, num_heads, num_kv_hea
         tensor_core = not general_only and k_cache is not v_cache and ops.scored_takes_tensor_cores(
             q.dtype, q.shape[1] // num_heads, v_dim, group_size, k_cache.shape[2], prompt=q_tile > 1)
         if not general_only and k_cache is v_cache and ops.shared_rows_take_tensor_cores(q.dtype, q.shape[1] // num_heads, v_dim):
-            splits = ops.choose_splits_shared_rows(hi - lo, num_kv_heads, q_tile * group_size, longest)
+            splits = ops.choose_splits_shared_rows(num_tiles, num_kv_heads, q_tile * group_size, longest)
         elif q_tile > 1 and tensor_core:
             splits = 1
         else:
-            splits = ops.choose_splits(hi - lo, num_kv_heads, q_tile * group_size, longest, tensor_core,
+            splits = ops.choose_splits(num_tiles, num_kv_heads, q_tile * group_size, longest, tensor_core,
                                        mean_context=mean)
         ops.scored_attention(
-            q, k_cache, v_cache, group.block_table, ctx.cu_q, ctx.ctx_lens, ctx.tile_seq[lo:hi], ctx.tile_q0[lo:hi],
-            ctx.tile_nq[lo:hi], num_tiles=hi - lo, q_tile=q_tile, num_splits=splits, num_heads=num_heads,
+            q, k_cache, v_cache, group.block_table, ctx.cu_q, ctx.ctx_lens, *tiles,
+            num_tiles=num_tiles, q_tile=q_tile, num_splits=splits, num_heads=num_heads,
             num_kv_heads=num_kv_heads, v_dim=v_dim, scale=scale, window=window, chunk=chunk, softcap=softcap,
             slopes=slopes, gate=gate, status=ctx.status, out=out, keep_first=keep_first,
             sigmoid_weights=sigmoid_weights, head_bias=head_bias, out_scale=out_scale, sink=sink)
