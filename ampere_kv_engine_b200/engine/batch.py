@@ -71,7 +71,9 @@ class StepContext:
     q_lens_host: list[int] = field(default_factory=list)
     ctx_lens_host: list[int] = field(default_factory=list)
     state_slots_host: list[int] = field(default_factory=list)
-    h2d_bytes: int = 0              # size of the one host-to-device copy that carried all of the above
+    h2d_bytes: int = 0              # size of the one host-to-device copy that carried all of the above and the extras
+    #: what parts laid out for this step beside the above, by their keys (``Part.step_extras``)
+    extras: dict = field(default_factory=dict)
     #: what one layer leaves for later layers of the same step, by name (values that a later mixer blends with its
     #: own, for instance); emptied when a step's forward pass begins
     shared: dict = field(default_factory=dict)
@@ -92,12 +94,14 @@ class BatchLayout:
     num_tiles: int
     widths: tuple[int, ...]           # block-table width per cache group
     offsets: list[int] = field(default_factory=list)
+    extras: tuple[int, ...] = ()      # sizes of what parts lay out beside the above
 
     def __post_init__(self):
         sizes = [self.num_tokens, self.num_tokens, self.num_seqs + 1, self.num_seqs, self.num_seqs,
                  max(1, self.num_logit_rows), self.num_tiles, self.num_tiles, self.num_tiles]
         for w in self.widths:
             sizes += [self.num_tokens, self.num_seqs * w]
+        sizes += self.extras
         self.offsets = [0]
         for size in sizes:
             self.offsets.append(self.offsets[-1] + _align(size))
@@ -107,6 +111,7 @@ class BatchLayout:
         return self.offsets[-1]
 
     def key(self) -> tuple:
+        """For layouts of decode steps, which have no extras."""
         return (self.num_tokens, self.num_seqs, self.num_logit_rows, self.num_tiles, self.widths)
 
 
@@ -174,7 +179,7 @@ def fill_host(manager: CacheManager, entries: list[SeqStep], layout: BatchLayout
 def make_context(layout: BatchLayout, dev: torch.Tensor, *, tile_rows: int, max_context: int,
                  status: torch.Tensor | None, q_lens: list[int], ctx_lens: list[int], state_slots: list[int],
                  h2d_bytes: int, sampled: torch.Tensor | None = None,
-                 decode_contexts: tuple[int, int] | None = None) -> StepContext:
+                 decode_contexts: tuple[int, int] | None = None, extras: dict | None = None) -> StepContext:
     """Views into the device copy ``dev`` of a filled index buffer."""
     off = layout.offsets
 
@@ -190,6 +195,8 @@ def make_context(layout: BatchLayout, dev: torch.Tensor, *, tile_rows: int, max_
     for gi, width in enumerate(layout.widths):
         groups.append(GroupBatch(view(9 + 2 * gi, layout.num_tokens),
                                  view(10 + 2 * gi, layout.num_seqs * width).view(layout.num_seqs, width), width))
+    first = 9 + 2 * len(layout.widths)
+    placed = {key: extra.place(view(first + i, layout.extras[i])) for i, (key, extra) in enumerate((extras or {}).items())}
     return StepContext(
         num_tokens=layout.num_tokens, num_seqs=layout.num_seqs, token_ids=view(0, layout.num_tokens),
         positions=view(1, layout.num_tokens), cu_q=view(2, layout.num_seqs + 1), ctx_lens=view(3, layout.num_seqs),
@@ -198,7 +205,7 @@ def make_context(layout: BatchLayout, dev: torch.Tensor, *, tile_rows: int, max_
         tile_nq=view(8, layout.num_tiles), num_tiles=layout.num_tiles, q_tile=tile_rows,
         num_decode_tiles=num_decode_tiles, max_context=max_context, decode_contexts=decode_contexts,
         groups=groups, status=status, sampled=sampled, q_lens_host=q_lens, ctx_lens_host=ctx_lens,
-        state_slots_host=state_slots, h2d_bytes=h2d_bytes)
+        state_slots_host=state_slots, h2d_bytes=h2d_bytes, extras=placed)
 
 
 def validate_entries(entries: list[SeqStep]) -> None:
@@ -216,28 +223,36 @@ def validate_entries(entries: list[SeqStep]) -> None:
                                  f"{len(e.tokens)} tokens")
 
 
-def exact_layout(manager: CacheManager, entries: list[SeqStep], tile_rows: int) -> BatchLayout:
+def exact_layout(manager: CacheManager, entries: list[SeqStep], tile_rows: int, extras: dict | None = None) -> BatchLayout:
     q_lens = [len(e.tokens) for e in entries]
     widths = tuple(max(1, max(len(manager.table_row(e.seq, g.index)) for e in entries)) for g in manager.groups)
     return BatchLayout(sum(q_lens), len(entries), sum(len(e.want) for e in entries),
-                       sum((n + tile_rows - 1) // tile_rows for n in q_lens), widths)
+                       sum((n + tile_rows - 1) // tile_rows for n in q_lens), widths,
+                       extras=tuple(len(extra.numbers) for extra in (extras or {}).values()))
 
 
 def build_context(manager: CacheManager, entries: list[SeqStep], device: torch.device,
                   status: torch.Tensor | None = None, q_tile: int | None = None,
-                  sampled: torch.Tensor | None = None) -> StepContext:
+                  sampled: torch.Tensor | None = None, step_extras=None) -> StepContext:
     """Lay out the step exactly (no padding) and copy it to the device in one transfer.  Every entry's pages
-    must already be reserved for its new tokens."""
+    must already be reserved for its new tokens.  ``step_extras`` (the model's; called for steps with prompt portions):
+    what its parts add to that transfer."""
     validate_entries(entries)
     q_tile = q_tile or ops.ATTENTION_Q_TILE
     tile_rows = 1 if max(len(e.tokens) for e in entries) == 1 else q_tile
-    layout = exact_layout(manager, entries, tile_rows)
+    extras = {}
+    if step_extras is not None and tile_rows > 1:
+        extras = step_extras([len(e.tokens) for e in entries], [e.seq.length + len(e.tokens) for e in entries], tile_rows)
+    layout = exact_layout(manager, entries, tile_rows, extras)
     host = np.empty(layout.total, dtype=np.int32)
     q_lens, ctx_lens = fill_host(manager, entries, layout, host, tile_rows)
+    for i, extra in enumerate(extras.values()):
+        at = layout.offsets[9 + 2 * len(layout.widths) + i]
+        host[at:at + len(extra.numbers)] = extra.numbers
     staged = torch.from_numpy(host)
     if device.type == "cuda":
         staged = staged.pin_memory()
     dev = staged.to(device, non_blocking=True)
     return make_context(layout, dev, tile_rows=tile_rows, max_context=max(ctx_lens), status=status, q_lens=q_lens,
                         ctx_lens=ctx_lens, state_slots=[e.seq.state_slot for e in entries], h2d_bytes=int(host.nbytes),
-                        sampled=sampled)
+                        sampled=sampled, extras=extras)

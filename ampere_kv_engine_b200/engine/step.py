@@ -122,7 +122,7 @@ class ModelRunner:
                 logits = self._decode_step_captured(entries)
             else:
                 ctx = build_context(self.manager, entries, self.device, status=self.status, sampled=self.sampled,
-                                    q_tile=self.q_tile)
+                                    q_tile=self.q_tile, step_extras=getattr(self.model, "step_extras", None))
                 self.last_h2d_bytes = ctx.h2d_bytes
                 logits = self.model.forward(ctx, self.views)
         except BaseException:

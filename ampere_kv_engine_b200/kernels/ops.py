@@ -557,9 +557,6 @@ class LatentStep:
         self.numbers = [v for plan in plans for v in plan.numbers] + [t[i] for i in range(3) for t in tiles]
         self.tiles = None
 
-    def to(self, device):
-        return self.place(torch.tensor(self.numbers, dtype=torch.int32).pin_memory().to(device, non_blocking=True))
-
     def place(self, numbers: torch.Tensor):
         """``numbers``: this object's numbers on the device."""
         at = 0

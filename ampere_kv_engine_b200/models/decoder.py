@@ -109,6 +109,13 @@ class DecoderModel:
                   if m is not None and m.preferred_q_tile() is not None}
         return wishes.pop() if len(wishes) == 1 else ops.ATTENTION_Q_TILE
 
+    def step_extras(self, q_lens: list[int], ctx_lens: list[int], q_tile: int) -> dict:
+        """What the parts want beside a step's index data (:meth:`~ampere_kv_engine_b200.parts.base.Part.step_extras`)."""
+        extras: dict = {}
+        for part in self._parts():
+            part.step_extras(extras, q_lens, ctx_lens, q_tile)
+        return {key: extra for key, extra in extras.items() if extra is not None}
+
     def cache_of(self) -> list[int | None]:
         own = [None] if self.embedding.cache_spec().state_shape else []
         return [e.cache_of for e in self.spec.schedule] + own

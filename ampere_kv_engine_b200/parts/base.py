@@ -127,6 +127,12 @@ class Part:
     def load(self, tensors: dict[str, torch.Tensor]) -> None:
         """Receive the tensors of :meth:`param_specs` (already on the device, cast per kind)."""
 
+    def step_extras(self, extras: dict, q_lens: list[int], ctx_lens: list[int], q_tile: int) -> None:
+        """Called for a step that holds prompt portions before its index data travels: a part that wants numbers of its
+        own beside them adds an object under a key that says what it depends on (parts alike share one; None: nothing in
+        this step).  The object's ``numbers`` (ints) go into the step's one copy and ``place(tensor)`` receives them as
+        int32 on the device; ``forward`` finds the object in ``ctx.extras``."""
+
     def children(self) -> tuple["Part", ...]:
         """Parts this part built for itself (a mixer's position encoding): the model asks them for tensors and for
         ``graph_safe`` as it asks the part itself."""

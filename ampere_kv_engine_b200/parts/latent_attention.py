@@ -18,7 +18,7 @@ keys and values written out: since ``q_unrot . (W_uk c) = (W_uk^T q_unrot) . c``
 space (one batched product per step) and attention runs over the rows as they are stored, every head reading the same
 row as its key and the row's first ``kv_rank`` elements as its value; the result per head is a mix of latents (times
 the head's gate), which ``W_uv`` turns into the head's output (one more batched product).  Prompt portions in bfloat16
-(:meth:`LatentAttention.written_out`) share their keys among enough queries to have them written out for the step: one
+(:meth:`LatentAttention.step_extras`) share their keys among enough queries to have them written out for the step: one
 product makes every head's keys and values of the rows they see, and attention runs over those (``ops.latent_prompt_attention``).  Between the first product
 and the attention stands one row-wise kernel (``ops.latent_prep``; with a query latent also ``ops.rotate_pairs`` behind
 the second product).
@@ -164,20 +164,24 @@ class LatentAttention(Mixer):
             # per head its key rows and its value rows: one product writes both out for a prompt
             self.w_kv = torch.cat((self.w_uk, tensors[n["uv"]].view(H, self.v_dim, self.kv_rank)), dim=1).flatten(0, 1)
 
-    def written_out(self, ctx):
-        """The step's ``ops.LatentStep`` if it has prompt portions that are better off with keys and values written out,
-        else None.  A key costs a portion 2 rank (dim + v_dim) operations a head once, and each (query, key) pair then 2
-        (dim + rot_dim + v_dim) instead of 2 (2 rank + rot_dim), on a faster kernel."""
-        if self.w_kv is None or not any(n > 1 for n in ctx.q_lens_host):
-            return None
-        row_bytes = self.num_heads * (self.head_dim + self.v_dim) * 2
-        key = ("latent_prompt", self.window, row_bytes)
-        if key not in ctx.shared:
-            step = ops.latent_step(ctx.q_lens_host, ctx.ctx_lens_host, window=self.window, portion=LATENT_PORTION,
-                                   row_bytes=row_bytes, q_tile=ctx.q_tile, group_bytes=ops.LATENT_PLAN_BYTES,
-                                   most_bytes=ops.LATENT_PLAN_BYTES)
-            ctx.shared[key] = None if step is None else step.to(self.device)
-        return ctx.shared[key]
+    def step_extras(self, extras, q_lens, ctx_lens, q_tile):
+        """The step's ``ops.LatentStep``, where it has prompt portions that are better off with keys and values written
+        out.  A key costs a portion 2 rank (dim + v_dim) operations a head once, and each (query, key) pair then 2 (dim +
+        rot_dim + v_dim) instead of 2 (2 rank + rot_dim), on a faster kernel."""
+        if self.w_kv is not None and self.written_out not in extras:
+            extras[self.written_out] = ops.latent_step(
+                q_lens, ctx_lens, window=self.window, portion=LATENT_PORTION, row_bytes=self.row_bytes, q_tile=q_tile,
+                group_bytes=ops.LATENT_PLAN_BYTES, most_bytes=ops.LATENT_PLAN_BYTES)
+
+    @property
+    def row_bytes(self) -> int:
+        """Bytes of one latent's keys and values written out."""
+        return self.num_heads * (self.head_dim + self.v_dim) * 2
+
+    @property
+    def written_out(self) -> tuple:
+        """The key of :meth:`step_extras`: mixers alike in it share one object."""
+        return ("latents written out", self.window, self.row_bytes)
 
     def forward(self, x, ctx, cache, residual=None):
         if cache.writes != self.own_kv:
@@ -201,7 +205,7 @@ class LatentAttention(Mixer):
                                  in_offset=D, out_offset=rank, factor=self.rotary_factor)
         else:
             q = x[:, :self.q_width]
-        step = self.written_out(ctx)
+        step = getattr(ctx, "extras", {}).get(self.written_out)
         out = torch.empty((tokens, H * self.v_dim), dtype=q.dtype, device=q.device)
         if step is None or step.rows:
             # in the latent space; where other portions go the other way, the batch rows up to the last one that stays

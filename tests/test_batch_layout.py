@@ -49,3 +49,35 @@ def test_decode_contexts_of_a_step_without_single_tokens_fall_back_to_the_longes
     manager.reserve(seq, 5)
     ctx = build_context(manager, entries, torch.device("cpu"), q_tile=8)
     assert ctx.num_decode_tiles == 0 and ctx.decode_contexts == (15, 15)
+
+
+class _Extra:
+    def __init__(self, numbers):
+        self.numbers, self.placed = numbers, None
+
+    def place(self, tensor):
+        self.placed = tensor.tolist()
+        return self
+
+
+def test_what_parts_add_travels_with_the_step():
+    manager = _manager()
+    seqs = [_held(manager, "a", 30), _held(manager, "b", 0)]
+    asked = []
+
+    def extras(q_lens, ctx_lens, q_tile):
+        asked.append((q_lens, ctx_lens, q_tile))
+        return {"x": _Extra([5, -7, 9]), ("y", 2): _Extra([1 << 30])}
+
+    def context(new):
+        entries = [SeqStep(s, [1] * n, [0]) for s, n in zip(seqs, new)]
+        for e in entries:
+            manager.reserve(e.seq, len(e.tokens))
+        return build_context(manager, entries, torch.device("cpu"), q_tile=8, step_extras=extras)
+
+    ctx = context([1, 12])
+    assert asked == [([1, 12], [31, 12], 8)]
+    assert {key: extra.placed for key, extra in ctx.extras.items()} == {"x": [5, -7, 9], ("y", 2): [1 << 30]}
+    # a step of single tokens asks nobody
+    ctx = context([1, 1])
+    assert len(asked) == 1 and ctx.extras == {}

@@ -4,6 +4,7 @@ whatever order they come in."""
 import pytest
 import torch
 
+import ligirax_util
 import sukalorn_util
 
 pytestmark = pytest.mark.gpu
@@ -66,3 +67,23 @@ def test_groups_one_after_the_other(monkeypatch):
     got, grouped, _ = _run(monkeypatch, 16, held, new, group_bytes=256 * 20 * 88 * 2)
     assert whole == grouped == [0, 2, 3, 4]
     assert float((got - want).norm() / want.norm()) < 2.0 ** -6
+
+
+def test_a_step_travels_in_one_copy(monkeypatch):
+    """The plans of two layers that differ in their windows go with the step's index data, and are counted."""
+    from ampere_kv_engine_b200.config.engine_config import EngineConfig
+    from ampere_kv_engine_b200.engine.batch import SeqStep
+    from ampere_kv_engine_b200.engine.engine import Engine
+
+    runner = Engine.from_pretrained(ligirax_util.model_folder("L3"), config=EngineConfig(dtype="bfloat16", num_pages=100)).runner
+    seqs = [runner.open(f"r{i}") for i in range(2)]
+    pins, sizes = torch.Tensor.pin_memory, []
+
+    def pin(tensor, *args, **kw):
+        sizes.append(tensor.numel() * tensor.element_size())
+        return pins(tensor, *args, **kw)
+
+    monkeypatch.setattr(torch.Tensor, "pin_memory", pin)
+    runner.step([SeqStep(seqs[0], list(range(40)), [39]), SeqStep(seqs[1], list(range(5)), [4])])
+    runner.raise_on_status()
+    assert len(sizes) == 1 and runner.last_h2d_bytes == sizes[0]
