@@ -497,8 +497,10 @@ def rotate_pairs(x, out, positions, inv_freq, *, heads, cols, rotary_dims, in_of
 
 
 LATENT_TILE = 128          # query tokens of a tile, keys of a block: a sequence's gathered rows are a multiple of it
-#: most bytes of keys and values that are written out at a time; a portion that needs more stays in the latent space
+#: most bytes of one portion's keys and values that are written out; a portion that needs more stays in the latent space
 LATENT_PLAN_BYTES = 1 << 30
+#: most bytes of several portions' keys and values at a time
+LATENT_GROUP_BYTES = 1 << 29
 
 
 class LatentPlan:
@@ -592,6 +594,17 @@ def latent_step(q_lens: list[int], ctx_lens: list[int], *, window: int, portion:
     return LatentStep([latent_plan(q_lens, ctx_lens, window, only) for only in groups], tiles, kept)
 
 
+def latent_space(step: LatentStep, *, row: int, width: int, dtype, device):
+    """Room for the largest group of a step: (gathered rows, their keys and values), used by the groups one after the
+    other; None where the device has no memory left for it."""
+    rows = max(plan.rows for plan in step.plans)
+    try:
+        return (torch.empty((rows, row), dtype=dtype, device=device),
+                torch.empty((rows, width), dtype=dtype, device=device))
+    except torch.OutOfMemoryError:
+        return None
+
+
 def latent_prompt_takes(dtype: torch.dtype, device, dim: int, rot_dim: int, v_dim: int, rank: int) -> bool:
     """Whether :func:`latent_prompt_attention` has a kernel for these widths."""
     return dtype == torch.bfloat16 and torch.device(device).type == "cuda" and \
@@ -599,15 +612,18 @@ def latent_prompt_takes(dtype: torch.dtype, device, dim: int, rot_dim: int, v_di
 
 
 def latent_prompt_attention(q, q_rows, cache, block_table, plan: LatentPlan, w_kv, out, *, heads, dim, rot_dim, v_dim,
-                            rank, scale, window=0, gate=None, sink=None, status=None):
+                            rank, scale, window=0, gate=None, sink=None, status=None, space=None):
     """Causal attention of the plan's prompt portions over latents, with every head's keys and values written out: the
     cache rows the portions see are gathered, ``w_kv`` [heads * (dim + v_dim), rank] makes keys and values of them, and
     each query tile walks those of its head.  ``q`` [tokens, heads * (dim + rot_dim) and more]: the unturned dims of each
     head; ``q_rows`` [tokens, heads * (rank + rot_dim)]: the turned ones behind the first ``rank`` columns.  Writes the
-    portions' rows of ``out`` [tokens, heads * v_dim]; ``gate`` and ``sink`` as for :func:`scored_attention`."""
-    latents = torch.empty((plan.rows, rank + rot_dim), dtype=cache.dtype, device=cache.device)
+    portions' rows of ``out`` [tokens, heads * v_dim]; ``gate`` and ``sink`` as for :func:`scored_attention`; ``space`` as
+    :func:`latent_space` gives it."""
+    if space is None:
+        space = (cache.new_empty((plan.rows, rank + rot_dim)), cache.new_empty((plan.rows, heads * (dim + v_dim))))
+    latents, kv = (t[:plan.rows] for t in space)
     ext().latent_gather(cache, block_table, plan.plan, latents, plan.num_seqs, rank, status)
-    kv = torch.nn.functional.linear(latents[:, :rank], w_kv)
+    torch.mm(latents[:, :rank], w_kv.t(), out=kv)
     ext().latent_prompt_attention(q, q_rows, kv, latents, out, plan.plan, plan.num_seqs, plan.num_tiles, heads, dim, rot_dim,
                                   v_dim, rank, int(window or 0), float(scale), gate, sink, status)
     _launched(2)

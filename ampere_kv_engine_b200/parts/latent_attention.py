@@ -158,7 +158,7 @@ class LatentAttention(Mixer):
         self.w_uk = tensors[n["uk"]].view(H, self.head_dim, self.kv_rank).contiguous()
         self.w_uv = tensors[n["uv"]].view(H, self.v_dim, self.kv_rank).transpose(1, 2).contiguous()
         self.w_o = tensors[n["out"]].contiguous()
-        self.w_kv = None
+        self.w_kv, self.most_bytes = None, ops.LATENT_PLAN_BYTES
         if ops.latent_prompt_takes(self.dtype, self.device, self.head_dim, self.rot_dim, self.v_dim, self.kv_rank) \
                 and self.scale > 0 and (self.q_width if self.q_rank else self.w_in.shape[0]) % 8 == 0:
             # per head its key rows and its value rows: one product writes both out for a prompt
@@ -171,7 +171,8 @@ class LatentAttention(Mixer):
         if self.w_kv is not None and self.written_out not in extras:
             extras[self.written_out] = ops.latent_step(
                 q_lens, ctx_lens, window=self.window, portion=LATENT_PORTION, row_bytes=self.row_bytes, q_tile=q_tile,
-                group_bytes=ops.LATENT_PLAN_BYTES, most_bytes=ops.LATENT_PLAN_BYTES)
+                group_bytes=min(ops.LATENT_GROUP_BYTES, self.most_bytes),
+                most_bytes=min(ops.LATENT_PLAN_BYTES, self.most_bytes))
 
     @property
     def row_bytes(self) -> int:
@@ -181,7 +182,7 @@ class LatentAttention(Mixer):
     @property
     def written_out(self) -> tuple:
         """The key of :meth:`step_extras`: mixers alike in it share one object."""
-        return ("latents written out", self.window, self.row_bytes)
+        return ("latents written out", self.window, self.row_bytes, self.most_bytes)
 
     def forward(self, x, ctx, cache, residual=None):
         if cache.writes != self.own_kv:
@@ -205,7 +206,14 @@ class LatentAttention(Mixer):
                                  in_offset=D, out_offset=rank, factor=self.rotary_factor)
         else:
             q = x[:, :self.q_width]
-        step = getattr(ctx, "extras", {}).get(self.written_out)
+        step, space = getattr(ctx, "extras", {}).get(self.written_out), None
+        if step is not None:
+            space = ops.latent_space(step, row=self.row, width=H * (D + self.v_dim), dtype=q.dtype, device=q.device)
+            if space is None:
+                # the cache and the weights have left too little: this step stays in the latent space, and the next one
+                # asks for half
+                self.most_bytes = max(plan.rows for plan in step.plans) * self.row_bytes // 2
+                step = None
         out = torch.empty((tokens, H * self.v_dim), dtype=q.dtype, device=q.device)
         if step is None or step.rows:
             # in the latent space; where other portions go the other way, the batch rows up to the last one that stays
@@ -221,7 +229,7 @@ class LatentAttention(Mixer):
         for plan in step.plans if step is not None else ():
             ops.latent_prompt_attention(q, q_row, rows, group.block_table, plan, self.w_kv, out, heads=H, dim=D, rot_dim=R,
                                         v_dim=self.v_dim, rank=rank, scale=self.scale, window=self.window, gate=gate,
-                                        sink=self.sink, status=ctx.status)
+                                        sink=self.sink, status=ctx.status, space=space)
         if residual is not None:
             summed = ops.linear_into_residual(out, self.w_o, residual, status=ctx.status)
             if summed is not None:

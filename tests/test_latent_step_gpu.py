@@ -27,7 +27,7 @@ def _run(monkeypatch, portion, held, new, group_bytes=None):
             runner.step([SeqStep(seqs[i], tokens[7 * i:7 * i + n], [])])
     monkeypatch.setattr(latent_attention, "LATENT_PORTION", portion)
     if group_bytes is not None:
-        monkeypatch.setattr(ops, "LATENT_PLAN_BYTES", group_bytes)
+        monkeypatch.setattr(ops, "LATENT_GROUP_BYTES", group_bytes)
     written, stayed = [], []
     attention, scored = ops.latent_prompt_attention, ops.scored_attention
 
@@ -87,3 +87,37 @@ def test_a_step_travels_in_one_copy(monkeypatch):
     runner.step([SeqStep(seqs[0], list(range(40)), [39]), SeqStep(seqs[1], list(range(5)), [4])])
     runner.raise_on_status()
     assert len(sizes) == 1 and runner.last_h2d_bytes == sizes[0]
+
+
+def test_a_step_without_room_for_keys_and_values(monkeypatch):
+    """An engine whose weights and cache leave no room for a portion's written-out keys and values works on in the latent
+    space, and asks for less from then on."""
+    from ampere_kv_engine_b200.config.engine_config import EngineConfig
+    from ampere_kv_engine_b200.engine.batch import SeqStep
+    from ampere_kv_engine_b200.engine.engine import Engine
+    from ampere_kv_engine_b200.parts import latent_attention
+
+    runner = Engine.from_pretrained(sukalorn_util.model_folder("S3"),
+                                    config=EngineConfig(dtype="bfloat16", num_pages=2200)).runner
+    tokens = torch.randint(0, 320, (16400,), generator=torch.Generator().manual_seed(1)).tolist()
+    seqs = [runner.open("a"), runner.open("b")]
+    monkeypatch.setattr(latent_attention, "LATENT_PORTION", 10 ** 9)
+    for lo in range(0, 16384, 2048):
+        for seq in seqs:
+            runner.step([SeqStep(seq, tokens[lo:lo + 2048], [])])
+    want = runner.step([SeqStep(seqs[0], tokens[16384:], [15])])
+    monkeypatch.undo()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    # a portion of 16 tokens has small activations, but 58 MB of keys and values of its 16,400 latents
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (24 << 20)) / total)
+    try:
+        got = runner.step([SeqStep(seqs[1], tokens[16384:], [15])])
+        torch.cuda.synchronize()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    runner.raise_on_status()
+    torch.testing.assert_close(got, want, atol=0, rtol=0)
+    mixer = next(p for p in runner.model._parts() if isinstance(p, latent_attention.LatentAttention))
+    assert mixer.most_bytes == 16512 * 20 * 88 * 2 // 2
