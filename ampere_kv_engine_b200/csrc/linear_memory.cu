@@ -111,19 +111,20 @@ __global__ void __launch_bounds__(256) linear_prep_kernel(LinearScanParams p, in
   }
 }
 
-// The output rows of a sequence that cannot be walked: zeros, those of them that are rows of the batch.
-__device__ void zero_rows(const LinearScanParams& p, int head, int slice, int64_t first, int64_t last) {
-  const int cols = min(kScanColumns, p.v_dim - slice * kScanColumns);
-  const int64_t begin = first > 0 ? first : 0, end = last < p.num_tokens ? last : p.num_tokens;
-  float* out = p.out + (int64_t)head * p.v_dim + slice * kScanColumns;
-  for (int64_t i = threadIdx.x; i < (end - begin) * cols; i += blockDim.x)
-    out[(begin + i / cols) * p.num_heads * p.v_dim + i % cols] = 0.f;
+// The output rows [first, last) of a sequence that cannot be walked, `cols` columns from `out` on: zeros, those of them that
+// are rows of the batch.
+__device__ __noinline__ void zero_rows(float* out, int64_t stride, int cols, int64_t first, int64_t last, int64_t num_tokens) {
+  const int64_t begin = first > 0 ? first : 0, end = last < num_tokens ? last : num_tokens;
+  for (int64_t i = threadIdx.x; i < (end - begin) * cols; i += blockDim.x) out[(begin + i / cols) * stride + i % cols] = 0.f;
 }
 
 // PRODUCERS == 0: the decode form.  PRODUCERS > 0: the prompt form with that many further threads that only copy
 // the next chunk from p.act into shared memory beside the walk of the current one.
+// The decode form streams the memories, and what carries that is blocks in flight: at 16 rows a thread stays below 129
+// registers, so that two blocks of 256 share an SM.  (Room for more registers, or operations on pairs of rows, cost it:
+// 128 requests of 16 heads of 128 x 128 162 us with 143 registers, 99 with pairs in 128, 94 so.)
 template <typename T, int MODE, int ROWS, int CHUNK, int PRODUCERS>
-__global__ void __launch_bounds__(256 + PRODUCERS, 1)
+__global__ void __launch_bounds__(256 + PRODUCERS)
 linear_scan_kernel(LinearScanParams p, int lanes, int slices) {
   constexpr int kRounds = scan_rounds(ROWS, PRODUCERS);
   constexpr bool kPrepared = MODE == kPlainDecay || MODE == kTokenDecay;     // no activation, float32 input
@@ -140,7 +141,8 @@ linear_scan_kernel(LinearScanParams p, int lanes, int slices) {
   const int n = p.cu_q[seq + 1] - t0;
   if (slot < 0 || n == 0) return;                      // a padded sequence: nothing is read or written
   if (!sequence_inside(t0, (int64_t)p.cu_q[seq + 1] - t0, p.num_tokens, slot, p.num_slots, p.status)) {
-    zero_rows(p, head, slice, t0, p.cu_q[seq + 1]);
+    zero_rows(p.out + (int64_t)head * DV + slice * kScanColumns, (int64_t)H * DV, min(kScanColumns, DV - slice * kScanColumns),
+              t0, p.cu_q[seq + 1], p.num_tokens);
     return;
   }
   const int tid = threadIdx.x;
@@ -165,10 +167,10 @@ linear_scan_kernel(LinearScanParams p, int lanes, int slices) {
 
   float* mem = p.state + (int64_t)slot * p.state_stride +
                ((int64_t)head * slices + slice) * ROWS * (int64_t)threads + col * lanes + sub;
-  float2 S[ROWS / 2];      // neighbouring rows in pairs: every operation on them is one on two
+  float S[ROWS];
   if (walker) {
 #pragma unroll
-    for (int r = 0; r < ROWS; r += 2) S[r / 2] = make_float2(mem[(int64_t)r * threads], mem[(int64_t)(r + 1) * threads]);
+    for (int r = 0; r < ROWS; ++r) S[r] = mem[(int64_t)r * threads];
   }
   const float decay = (MODE == kConstantDecay || MODE == kPlainDecay) ? p.decay[head] : 0.f;
 
@@ -269,22 +271,29 @@ linear_scan_kernel(LinearScanParams p, int lanes, int slices) {
   };
   // a token's q, a and v applied to this thread's rows of S; returns its part of the token's output
   auto apply_loaded = [&](const float4 (&qs)[ROWS / 4], const float4 (&as)[ROWS / 4], float v, float decay) -> float {
-    float2 o01 = make_float2(0.f, 0.f), o23 = o01;
-    const float2 vv = make_float2(v, v), minus = make_float2(-v, -v), dd = make_float2(decay, decay);
-    auto step = [&](float2 old, float2 a) -> float2 {
-      // f S + (1 - f) v as v + f (S - v); the others k v + decay S
-      if (MODE == kGatedWrite) return fma2(a, add2(old, minus), vv);
-      return fma2(a, vv, mul2(dd, old));
-    };
+    float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
 #pragma unroll
     for (int r4 = 0; r4 < ROWS / 4; ++r4) {
       const float4 q = qs[r4], a = as[r4];
-      S[2 * r4] = step(S[2 * r4], make_float2(a.x, a.y));
-      S[2 * r4 + 1] = step(S[2 * r4 + 1], make_float2(a.z, a.w));
-      o01 = fma2(S[2 * r4], make_float2(q.x, q.y), o01);
-      o23 = fma2(S[2 * r4 + 1], make_float2(q.z, q.w), o23);
+      const int r = r4 * 4;
+      if (MODE == kGatedWrite) {
+        // f S + (1 - f) v as v + f (S - v): two operations per entry
+        S[r] = fmaf(a.x, S[r] - v, v);
+        S[r + 1] = fmaf(a.y, S[r + 1] - v, v);
+        S[r + 2] = fmaf(a.z, S[r + 2] - v, v);
+        S[r + 3] = fmaf(a.w, S[r + 3] - v, v);
+      } else {
+        S[r] = fmaf(a.x, v, decay * S[r]);
+        S[r + 1] = fmaf(a.y, v, decay * S[r + 1]);
+        S[r + 2] = fmaf(a.z, v, decay * S[r + 2]);
+        S[r + 3] = fmaf(a.w, v, decay * S[r + 3]);
+      }
+      o0 = fmaf(S[r], q.x, o0);
+      o1 = fmaf(S[r + 1], q.y, o1);
+      o2 = fmaf(S[r + 2], q.z, o2);
+      o3 = fmaf(S[r + 3], q.w, o3);
     }
-    return (o01.x + o01.y) + (o23.x + o23.y);
+    return (o0 + o1) + (o2 + o3);
   };
   // a token's row of [q | a | v] in shared memory into registers
   auto fetch = [&](const float* row, float4 (&qs)[ROWS / 4], float4 (&as)[ROWS / 4], float& v, float& d) {
@@ -375,10 +384,7 @@ linear_scan_kernel(LinearScanParams p, int lanes, int slices) {
   }
   if (walker) {
 #pragma unroll
-    for (int r = 0; r < ROWS; r += 2) {
-      mem[(int64_t)r * threads] = S[r / 2].x;
-      mem[(int64_t)(r + 1) * threads] = S[r / 2].y;
-    }
+    for (int r = 0; r < ROWS; ++r) mem[(int64_t)r * threads] = S[r];
   }
 }
 
@@ -408,7 +414,8 @@ __global__ void __launch_bounds__(RL * 8) linear_walk_kernel(LinearScanParams p,
   const int n = p.cu_q[seq + 1] - first;
   if (slot < 0 || n == 0) return;                      // a padded sequence: nothing is read or written
   if (!sequence_inside(first, (int64_t)p.cu_q[seq + 1] - first, p.num_tokens, slot, p.num_slots, p.status)) {
-    zero_rows(p, head, slice, first, p.cu_q[seq + 1]);
+    zero_rows(p.out + (int64_t)head * DV + slice * kScanColumns, (int64_t)H * DV, min(kScanColumns, DV - slice * kScanColumns),
+              first, p.cu_q[seq + 1], p.num_tokens);
     return;
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
