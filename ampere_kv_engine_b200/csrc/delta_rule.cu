@@ -427,8 +427,12 @@ __global__ void __launch_bounds__(RL * 8) delta_walk_kernel(DeltaParams p, int e
   extern __shared__ __align__(16) float smem[];
   pdl_launch_dependents();
   pdl_wait();
-  const int s = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * kWalkColumns;
   const int G = p.num_kv_heads, H = p.num_heads, D = p.head_dim, V = p.v_dim;
+  // A sequence's blocks are neighbours, so that a long one's fall on different SMs, and the last sequence comes first: a
+  // batch holds its prompt portions behind its single tokens, and the longest walk should not begin last.
+  const int slices = (V + kWalkColumns - 1) / kWalkColumns;
+  const int col0 = (int)(blockIdx.x % slices) * kWalkColumns, h = (int)(blockIdx.x / slices) % H;
+  const int s = p.num_seqs - 1 - (int)(blockIdx.x / slices) / H;
   const int channels = 2 * G * D + H * V;
   const int64_t first = p.cu_q[s];
   const int n = (int)(p.cu_q[s + 1] - first);
@@ -689,9 +693,9 @@ static int launch_walk(const DeltaParams& p, const ScanShape& shape, cudaStream_
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return (int)err;
   }
-  const int slices = (p.v_dim + kWalkColumns - 1) / kWalkColumns;
-  return (int)launch_alone(kernel, dim3((unsigned)p.num_seqs, (unsigned)p.num_heads, (unsigned)slices), dim3(RL * 8), smem,
-                           stream, p, shape.ept, shape.lanes);
+  const int64_t blocks = (int64_t)p.num_seqs * p.num_heads * ((p.v_dim + kWalkColumns - 1) / kWalkColumns);
+  if (blocks > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
+  return (int)launch_alone(kernel, dim3((unsigned)blocks), dim3(RL * 8), smem, stream, p, shape.ept, shape.lanes);
 }
 
 template <int EPT, int LANES, int CHUNK, bool CHANNEL>

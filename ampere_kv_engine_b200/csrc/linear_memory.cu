@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(RL * 8) linear_walk_kernel(LinearScanParams p,
   const int H = p.num_heads, D = p.head_dim, DV = p.v_dim;
   const int slice = blockIdx.x % slices;
   const int head = (blockIdx.x / slices) % H;
-  const int seq = blockIdx.x / (slices * H);
+  const int seq = p.num_seqs - 1 - blockIdx.x / (slices * H);      // prompt portions, which are a batch's last, begin first
   const int slot = p.state_slots[seq];
   const int first = p.cu_q[seq];
   const int n = p.cu_q[seq + 1] - first;
