@@ -416,8 +416,8 @@ __global__ void __launch_bounds__(256) delta_scan_kernel(DeltaParams p, int cols
 // 16 numbers serve 32 elements.  What a token needs of S, S^T k, and what the token before it is read out with, S^T q, are
 // taken from the same S: eight sums, which go through ONE exchange over RL lanes.  A token's numbers stand in registers one
 // token ahead; tokens arrive kWalkChunk at a time by asynchronous copies, a warp a token.  16 heads of 128 x 128 (us, before | now):
-// one sequence of 2,048 tokens 640 | 575, three of 1,501, 301 and 246 556 | 554, seven of 300 398 | 206; 32 heads 656 | 591,
-// 855 | 724, 695 | 349.
+// one sequence of 2,048 tokens 635 | 494, three of 1,501, 301 and 246 550 | 383, seven of 300 393 | 185; 32 heads 654 | 511,
+// 849 | 525, 696 | 316.
 template <int RL, int QUADS, bool CHANNEL>
 __global__ void __launch_bounds__(RL * 8) delta_walk_kernel(DeltaParams p, int ept, int lanes) {
   constexpr int kRowsPadded = RL * 4 * QUADS, kPairs = 2 * QUADS, kChunk = kWalkChunk, kWarps = RL / 4;
@@ -428,11 +428,10 @@ __global__ void __launch_bounds__(RL * 8) delta_walk_kernel(DeltaParams p, int e
   pdl_launch_dependents();
   pdl_wait();
   const int G = p.num_kv_heads, H = p.num_heads, D = p.head_dim, V = p.v_dim;
-  // A sequence's blocks are neighbours, so that a long one's fall on different SMs, and the last sequence comes first: a
-  // batch holds its prompt portions behind its single tokens, and the longest walk should not begin last.
+  // a sequence's blocks are neighbours, so that a long one's fall on different SMs
   const int slices = (V + kWalkColumns - 1) / kWalkColumns;
   const int col0 = (int)(blockIdx.x % slices) * kWalkColumns, h = (int)(blockIdx.x / slices) % H;
-  const int s = p.num_seqs - 1 - (int)(blockIdx.x / slices) / H;
+  const int s = sequence_in_turn(p.cu_q, p.num_seqs, (int)(blockIdx.x / slices) / H);
   const int channels = 2 * G * D + H * V;
   const int64_t first = p.cu_q[s];
   const int n = (int)(p.cu_q[s + 1] - first);
@@ -573,9 +572,13 @@ __global__ void __launch_bounds__(RL * 8) delta_walk_kernel(DeltaParams p, int e
 #pragma unroll
     for (int r = 0; r < kPairs; ++r) read[r] = x.q[r];
   };
-  // rows beyond the dim and columns beyond the width stay zero in both buffers
-  for (int i = threadIdx.x; i < (2 * kChunk + 1) * kToken; i += blockDim.x) smem[i] = 0.f;
-  __syncthreads();
+  // rows beyond the dim and columns beyond the width stay zero in both buffers; nothing else needs a value before a token
+  // arrives, so buffers of whole heads are not filled
+  const int rows_over = kRowsPadded - D, over = kVecs * rows_over + kWalkColumns - mine_cols;
+  for (int i = threadIdx.x; i < 2 * kChunk * over; i += blockDim.x) {
+    const int t = i / over, e = i - t * over, vec = rows_over > 0 ? min(e / rows_over, kVecs) : kVecs;
+    smem[t * kToken + vec * kRowsPadded + (vec < kVecs ? D : mine_cols) + (e - vec * rows_over)] = 0.f;
+  }
   copy(smem, 0, min(kChunk, n));
   copy_async_wait_all();
   __syncthreads();
@@ -695,6 +698,8 @@ static int launch_walk(const DeltaParams& p, const ScanShape& shape, cudaStream_
   }
   const int64_t blocks = (int64_t)p.num_seqs * p.num_heads * ((p.v_dim + kWalkColumns - 1) / kWalkColumns);
   if (blocks > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
+  if (p.num_tokens - p.num_seqs <= kShortWalk)
+    return (int)launch_chain(kernel, dim3((unsigned)blocks), dim3(RL * 8), smem, stream, dim3(1, 1, 1), p, shape.ept, shape.lanes);
   return (int)launch_alone(kernel, dim3((unsigned)blocks), dim3(RL * 8), smem, stream, p, shape.ept, shape.lanes);
 }
 

@@ -241,13 +241,16 @@ linear_scan_kernel(LinearScanParams p, int lanes, int slices) {
       }
     }
   };
-  // the same from the scratch that the preparing kernel filled (prompt form): asynchronous copies, all of a chunk in
-  // flight at once
+  // the same from the scratch that the preparing kernel filled (prompt form): asynchronous copies of 16 bytes where
+  // the widths allow it, of 4 otherwise, all of a chunk in flight at once
   auto stage_copy = [&](float* buffer, int first, int count) {
     const int64_t width = p.act_stride;
+    const bool wide_copy = D % 4 == 0 && DV % 4 == 0 && p.act_aligned;
+    const int step = wide_copy ? 4 : 1;
+    const int per = fetch_per_token / step;
     const float* base = p.act + (int64_t)(t0 + first) * width;
-    for (int e = stage_id; e < count * fetch_per_token; e += stagers) {
-      const int t = e / fetch_per_token, i = e % fetch_per_token;
+    for (int e = stage_id; e < count * per; e += stagers) {
+      const int t = e / per, i = (e % per) * step;
       const float* from = base + (int64_t)t * width;
       float* to = buffer + t * per_token;
       if (i < D) {
@@ -260,7 +263,8 @@ linear_scan_kernel(LinearScanParams p, int lanes, int slices) {
         from += p.act_v_off + head * DV + slice * kScanColumns + (i - 2 * D);
         to += 2 * vec + (i - 2 * D);
       }
-      copy_async<4>(to, from);
+      if (wide_copy) copy_async<16>(to, from);
+      else copy_async<4>(to, from);
     }
     if (MODE == kTokenDecay) {
       for (int t = stage_id; t < count; t += stagers)
@@ -394,11 +398,13 @@ linear_scan_kernel(LinearScanParams p, int lanes, int slices) {
 // elements; RL lanes x 4 QUADS rows cover the dim, a block again 32 columns.  The outputs of two tokens, eight sums, go
 // through one exchange over RL lanes.  A token's numbers stand in registers one token ahead; tokens arrive kWalkChunk at a
 // time by asynchronous copies, a warp a token.  Forget gates, 16 heads of 128 x 128 (us, before | now, with the preparation):
-// one sequence of 2,048 tokens 394 | 326, two of 1,024 232 | 181, seven of 300 281 | 152; 32 heads 458 | 345, 464 | 269,
-// 509 | 251.
+// one sequence of 2,048 tokens 390 | 310, two of 1,024 226 | 169, seven of 300 277 | 150; 32 heads 453 | 327, 459 | 253,
+// 505 | 249; 64 of four tokens each 387 | 165.
 constexpr int kWalkChunk = 16;
-template <int MODE, int RL, int QUADS>
-__global__ void __launch_bounds__(RL * 8) linear_walk_kernel(LinearScanParams p, int rows, int lanes, int slices) {
+// DENSE: registers for more blocks an SM (five of 128 threads, ten of 64), which many short sequences want; otherwise for
+// the shortest chain of a token (launch_scan says which).
+template <int MODE, int RL, int QUADS, bool DENSE>
+__global__ void __launch_bounds__(RL * 8, DENSE ? (RL == 16 ? 5 : (RL == 8 ? 10 : 2)) : 2) linear_walk_kernel(LinearScanParams p, int rows, int lanes, int slices) {
   constexpr int kRowsPadded = RL * 4 * QUADS, kPairs = 2 * QUADS, kWarps = RL / 4;
   constexpr int kToken = 2 * kRowsPadded + kScanColumns + (MODE == kTokenDecay ? 4 : 0);       // [q | a | v (| decay)]
   constexpr int kPieces = (2 * kRowsPadded + kScanColumns + 127) / 128;
@@ -408,7 +414,7 @@ __global__ void __launch_bounds__(RL * 8) linear_walk_kernel(LinearScanParams p,
   const int H = p.num_heads, D = p.head_dim, DV = p.v_dim;
   const int slice = blockIdx.x % slices;
   const int head = (blockIdx.x / slices) % H;
-  const int seq = p.num_seqs - 1 - blockIdx.x / (slices * H);      // prompt portions, which are a batch's last, begin first
+  const int seq = sequence_in_turn(p.cu_q, p.num_seqs, blockIdx.x / (slices * H));
   const int slot = p.state_slots[seq];
   const int first = p.cu_q[seq];
   const int n = p.cu_q[seq + 1] - first;
@@ -423,20 +429,25 @@ __global__ void __launch_bounds__(RL * 8) linear_walk_kernel(LinearScanParams p,
   const int mine_cols = min(kScanColumns, DV - slice * kScanColumns);
   const int qk_head = head / p.qk_group;
   const float decay = (MODE == kConstantDecay || MODE == kPlainDecay) ? p.decay[head] : 0.f;
-  // row i of the thread's: 4 RL (i / 4) + 4 rl + i % 4, and where it lies in the state slot
-  float* memory = p.state + (int64_t)slot * p.state_stride + ((int64_t)head * slices + slice) * rows * kScanColumns * lanes;
+  // The block's slice of the state slot is one run of numbers ([row in lane][column][lane]), but a thread's own are
+  // scattered over it: it travels in whole lines through the second token buffer (four numbers more behind every fourth
+  // row, so that the threads' accesses there spread over the banks).
+  const int slice_floats = rows * kScanColumns * lanes, row_floats = kScanColumns * lanes;
+  float* memory = p.state + (int64_t)slot * p.state_stride + ((int64_t)head * slices + slice) * slice_floats;
+  float* staged = smem + kWalkChunk * kToken;
+  const bool whole = (reinterpret_cast<uintptr_t>(memory) & 15) == 0;
+  auto staged_at = [&](int i) -> float* { return staged + i + (i / (4 * row_floats)) * 4; };
+  if (whole) {
+    for (int i = threadIdx.x * 4; i < slice_floats; i += blockDim.x * 4) copy_async<16>(staged_at(i), memory + i);
+  } else {
+    for (int i = threadIdx.x; i < slice_floats; i += blockDim.x) copy_async<4>(staged_at(i), memory + i);
+  }
+  // row i of the thread's, 4 RL (i / 4) + 4 rl + i % 4, in the staged slice
   auto place = [&](int i, int c) -> float* {
-    const int d = (i >> 2) * 4 * RL + 4 * rl + (i & 3);
-    return d < rows * lanes ? memory + ((int64_t)(d % rows) * kScanColumns + col + c) * lanes + d / rows : nullptr;
+    const int d = (i >> 2) * 4 * RL + 4 * rl + (i & 3), r = d % rows;
+    return d < rows * lanes ? staged + (r * kScanColumns + col + c) * lanes + d / rows + (r >> 2) * 4 : nullptr;
   };
   float2 S[kPairs][4];                                 // [pair of rows][column]
-#pragma unroll
-  for (int r = 0; r < kPairs; ++r)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const float *a = place(2 * r, c), *b = place(2 * r + 1, c);
-      S[r][c] = make_float2(a != nullptr ? *a : 0.f, b != nullptr ? *b : 0.f);
-    }
   int piece_from[kPieces], piece_to[kPieces];
 #pragma unroll
   for (int r = 0; r < kPieces; ++r) {
@@ -509,15 +520,30 @@ __global__ void __launch_bounds__(RL * 8) linear_walk_kernel(LinearScanParams p,
     if (stores && (both || !second)) to[(second ? wide : 0) + own] = o;
   };
   // rows of S beyond the dim never change: q and k stay zero there, a forget gate one; value columns beyond the width
-  // stay zero
-  for (int i = threadIdx.x; i < (2 * kWalkChunk + 1) * kToken; i += blockDim.x) {
-    const int e = i % kToken;
-    smem[i] = (MODE == kGatedWrite && e >= kRowsPadded && e < 2 * kRowsPadded) ? 1.f : 0.f;
-  }
-  __syncthreads();
+  // stay zero.  Nothing else needs a value before a token arrives, so buffers of whole heads are not filled.
+  auto fill = [&](float* buffer) {
+    const int rows_over = kRowsPadded - D, over = 2 * rows_over + kScanColumns - mine_cols;
+    if (over == 0) return;
+    for (int i = threadIdx.x; i < kWalkChunk * over; i += blockDim.x) {
+      const int t = i / over, e = i - t * over;
+      const int at = e < rows_over ? D + e : (e < 2 * rows_over ? kRowsPadded + D + (e - rows_over)
+                                                                : 2 * kRowsPadded + mine_cols + (e - 2 * rows_over));
+      buffer[t * kToken + at] = MODE == kGatedWrite && e >= rows_over && e < 2 * rows_over ? 1.f : 0.f;
+    }
+  };
+  fill(smem);
   copy(smem, 0, min(kWalkChunk, n));
   copy_async_wait_all();
   __syncthreads();
+#pragma unroll
+  for (int r = 0; r < kPairs; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float *a = place(2 * r, c), *b = place(2 * r + 1, c);
+      S[r][c] = make_float2(a != nullptr ? *a : 0.f, b != nullptr ? *b : 0.f);
+    }
+  __syncthreads();                                     // the second buffer is free for tokens
+  fill(staged);
   const int64_t wide = (int64_t)H * DV;
   float* out = p.out + (int64_t)first * wide + (int64_t)head * DV + slice * kScanColumns;
   for (int c0 = 0; c0 < n; c0 += kWalkChunk) {
@@ -551,6 +577,7 @@ __global__ void __launch_bounds__(RL * 8) linear_walk_kernel(LinearScanParams p,
     copy_async_wait_all();
     __syncthreads();
   }
+  // (behind the last chunk's barrier: no token is read any more)
 #pragma unroll
   for (int r = 0; r < kPairs; ++r)
 #pragma unroll
@@ -559,6 +586,13 @@ __global__ void __launch_bounds__(RL * 8) linear_walk_kernel(LinearScanParams p,
       if (a != nullptr) *a = S[r][c].x;
       if (b != nullptr) *b = S[r][c].y;
     }
+  __syncthreads();
+  if (whole) {
+    for (int i = threadIdx.x * 4; i < slice_floats; i += blockDim.x * 4)
+      *reinterpret_cast<float4*>(memory + i) = *reinterpret_cast<const float4*>(staged_at(i));
+  } else {
+    for (int i = threadIdx.x; i < slice_floats; i += blockDim.x) memory[i] = *staged_at(i);
+  }
 }
 
 // v[t, c]   = in[t, c] (+ skip_coef[c / skip_head] * skip[t, skip_off + c])  (* gate(x[t, gate_off + c]), gate_first)
@@ -706,17 +740,19 @@ static int launch_scan_chunk(const LinearScanParams& p, int lanes, cudaStream_t 
                            dim3(1, 1, 1), p, lanes, slices);
 }
 
-template <int MODE, int RL, int QUADS>
+template <int MODE, int RL, int QUADS, bool DENSE>
 static int launch_walk(const LinearScanParams& p, int rows, int lanes, cudaStream_t stream) {
   const int slices = (p.v_dim + kScanColumns - 1) / kScanColumns;
   const int64_t blocks = (int64_t)p.num_seqs * p.num_heads * slices;
   if (blocks > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
   const size_t smem = (2 * (size_t)kWalkChunk + 1) * (2 * RL * 4 * QUADS + kScanColumns + (MODE == kTokenDecay ? 4 : 0)) * sizeof(float);
-  auto kernel = linear_walk_kernel<MODE, RL, QUADS>;
+  auto kernel = linear_walk_kernel<MODE, RL, QUADS, DENSE>;
   if (smem > 48 * 1024) {
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return (int)err;
   }
+  if (p.num_tokens - p.num_seqs <= kShortWalk)
+    return (int)launch_chain(kernel, dim3((unsigned)blocks), dim3(RL * 8), smem, stream, dim3(1, 1, 1), p, rows, lanes, slices);
   return (int)launch_alone(kernel, dim3((unsigned)blocks), dim3(RL * 8), smem, stream, p, rows, lanes, slices);
 }
 
@@ -742,12 +778,25 @@ static int launch_scan(const LinearScanParams& p, int lanes, cudaStream_t stream
                                 : launch_chain(linear_prep_kernel<T, MODE, 1>, grid, dim3(256), 0, stream, dim3(1, 1, 1), p, width));
     if (err != 0) return err;
   }
-  if (p.head_dim % 4 == 0 && p.v_dim % 4 == 0 && p.act_aligned) {
+  // `extra` tokens at most stand behind a sequence's first.  Where a few blocks walk a short way the scan with staging warps
+  // needs less to begin with (us, forget gates, this | the walk: 16 heads of 64 x 64, 33 tokens 12.9 | 15.6, 100 tokens 21.5 |
+  // 25.2, 200 tokens 35 to 43 | 35.6; 16 heads of 128 x 128, 33 tokens 16.8 | 18.2, 100 tokens 28.4 | 27.5, twice 64 23.3 |
+  // 23.2, four times 64 43.8 | 29.4).
+  const int64_t extra = p.num_tokens - p.num_seqs;
+  const int64_t blocks = (int64_t)p.num_seqs * p.num_heads * ((p.v_dim + kScanColumns - 1) / kScanColumns);
+  const bool few = p.head_dim <= 64 ? blocks <= 2 * sm_count() && extra <= 128
+                                    : p.head_dim <= 128 && blocks <= sm_count() && extra <= 64;
+  if (p.head_dim % 4 == 0 && p.v_dim % 4 == 0 && p.act_aligned && !few) {
+    // Many blocks on short ways are carried by blocks in flight, few or long ones by the chain of a token (us, forget gates,
+    // dense | not: 16 heads of 128 x 128, 64 times four tokens 86 | 113, one sequence of 2,048 354 | 309; 16 heads of 64 x 64
+    // 27.5 | 35.9, 339 | 236).
+    const bool dense = blocks > 2 * sm_count() && extra <= 256;
     if constexpr (ROWS == 16) {
-      if (p.head_dim <= 64) return launch_walk<MODE, 8, 2>(p, ROWS, lanes, stream);
-      return launch_walk<MODE, 16, 2>(p, ROWS, lanes, stream);
+      if (p.head_dim <= 64)
+        return dense ? launch_walk<MODE, 8, 2, true>(p, ROWS, lanes, stream) : launch_walk<MODE, 8, 2, false>(p, ROWS, lanes, stream);
+      return dense ? launch_walk<MODE, 16, 2, true>(p, ROWS, lanes, stream) : launch_walk<MODE, 16, 2, false>(p, ROWS, lanes, stream);
     } else {
-      return launch_walk<MODE, 32, 2>(p, ROWS, lanes, stream);
+      return launch_walk<MODE, 32, 2, false>(p, ROWS, lanes, stream);
     }
   }
   return launch_scan_chunk<T, MODE, ROWS, (ROWS >= 32 ? 8 : 32), kScanProducers>(p, lanes, stream);
