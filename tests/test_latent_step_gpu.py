@@ -112,10 +112,16 @@ def test_a_step_without_room_for_keys_and_values(monkeypatch):
     # a portion of 16 tokens has small activations, but 58 MB of keys and values of its 16,400 latents
     total = torch.cuda.get_device_properties(0).total_memory
     torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (24 << 20)) / total)
+    taken = []
     try:
+        # what the process has reserved earlier and not given back must not hold them either
+        with pytest.raises(torch.OutOfMemoryError):
+            while True:
+                taken.append(torch.empty(32 << 20, dtype=torch.uint8, device="cuda"))
         got = runner.step([SeqStep(seqs[1], tokens[16384:], [15])])
         torch.cuda.synchronize()
     finally:
+        taken.clear()
         torch.cuda.set_per_process_memory_fraction(1.0)
     runner.raise_on_status()
     torch.testing.assert_close(got, want, atol=0, rtol=0)
