@@ -1,6 +1,6 @@
 """The routed experts' products on tcgen05 tiles: runs at the edges of the row tiles (1, 16, 17, 256, 257, 513 rows of
 one expert, an expert without rows), K and feature counts that end inside a block or a tile, choices that are no
-expert's."""
+expert's, several tiles for every CTA."""
 
 import pytest
 import torch
@@ -22,7 +22,11 @@ def _case(counts, k, n, top, form, seed=0):
 
 @pytest.mark.parametrize("form", ["gated", "up", "down"])
 @pytest.mark.parametrize("counts,k,n", [([1, 0, 3], 64, 1), ([16, 17, 1], 72, 130), ([256, 0, 257], 200, 128),
-                                        ([513, 40], 136, 257), ([5000], 64, 40)])
+                                        ([513, 40], 136, 257), ([5000], 64, 40),
+                                        # three to eight tiles a CTA, with ten K blocks each, which leave the ring (of
+                                        # three stages; of six) at another place and phase after every tile
+                                        ([37 * e % 600 + 1 for e in range(40)], 584, 1300),
+                                        ([5 * e % 17 for e in range(80)], 584, 1300)])
 def test_products_at_the_edges_of_the_tiles(form, counts, k, n):
     from ampere_kv_engine_b200.kernels import ops
 
