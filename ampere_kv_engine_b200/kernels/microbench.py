@@ -328,7 +328,7 @@ def bench_experts(args) -> dict:
     order, offsets = ops.moe_sort(chosen, E)
     used = int((offsets[1:] > offsets[:-1]).sum())
     out = {"experts_with_rows": used}
-    forms = ("few", "mma", "plain") if n * top <= 512 else ("mma",)
+    forms = ("tc", "few", "mma", "plain") if n * top <= 512 else ("tc", "mma")
     for form in forms:
         act = ops.moe_gate_up(x, w_gu[0], order, offsets, top=top, limit=7.0, slope=1.702, kernel=form)
         up_us = timed(lambda i: ops.moe_gate_up(x, w_gu[i % copies], order, offsets, top=top, limit=7.0, slope=1.702,

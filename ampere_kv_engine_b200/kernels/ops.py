@@ -506,9 +506,9 @@ LATENT_GROUP_BYTES = 1 << 29
 class LatentPlan:
     """Which keys of which sequences a step's prompt portions see (``csrc/launchers.h`` describes ``numbers``)."""
 
-    def __init__(self, numbers: list[int], num_seqs: int, num_tiles: int, rows: int, tokens: int, pairs: int):
+    def __init__(self, numbers: list[int], num_seqs: int, num_tiles: int, rows: int, tokens: int):
         self.numbers, self.num_seqs, self.num_tiles, self.rows = numbers, num_seqs, num_tiles, rows
-        self.tokens, self.pairs = tokens, pairs      # new tokens; (new token, key its sequence can see) pairs
+        self.tokens = tokens                         # new tokens
         self.plan = None
 
     def to(self, device):
@@ -526,7 +526,7 @@ def _latent_rows(n: int, c: int, window: int) -> tuple[int, int]:
 def latent_plan(q_lens: list[int], ctx_lens: list[int], window: int, only: set[int] | None = None) -> LatentPlan | None:
     """The plan of the sequences with more than one new token (of those in ``only``, if given; None without any): host
     lengths in, tiles with the most keys first."""
-    numbers, tiles, rows, row0, tokens, pairs = [], [], 0, 0, 0, 0
+    numbers, tiles, rows, row0, tokens = [], [], 0, 0, 0
     for s, (n, c) in enumerate(zip(q_lens, ctx_lens)):
         if n > 1 and (only is None or s in only):
             first, gathered = _latent_rows(n, c, window)
@@ -534,7 +534,6 @@ def latent_plan(q_lens: list[int], ctx_lens: list[int], window: int, only: set[i
             numbers += [rows, first, c, n, row0, s]
             rows += gathered
             tokens += n
-            pairs += n * (c - first)
             for t in range(0, n, LATENT_TILE):
                 last = c - n + min(n, t + LATENT_TILE)
                 tiles.append((last - max(first, c - n + t - window + 1 if window else 0), index, t))
@@ -545,7 +544,7 @@ def latent_plan(q_lens: list[int], ctx_lens: list[int], window: int, only: set[i
     count = len(numbers) // 6
     for _, index, t in tiles:
         numbers += [index, t]
-    return LatentPlan(numbers, count, len(tiles), rows, tokens, pairs)
+    return LatentPlan(numbers, count, len(tiles), rows, tokens)
 
 
 class LatentStep:
