@@ -20,14 +20,15 @@
 //   activations, gates).
 //   Prompt forms (everything else): a kernel of its own first writes every token's q, a-or-k and v after activations
 //   and gates as float32 (once per token, not once per block of a head's value slices).  Where the heads' rows are whole
-//   16-byte pieces, linear_walk_kernel then walks them in register tiles; otherwise in the scan a warp holds
+//   16-byte pieces, linear_walk_kernel then walks them in register tiles; otherwise, and where a few blocks walk a short
+//   way (launch_scan says which), in the scan a warp holds
 //   the same rows of all 32 columns, so its reads of q and of the gates are broadcasts; it leaves its part of every
 //   token's output in shared memory, and when the chunk is walked the walking warps add the parts up, a thread per
 //   (token, column).  Further warps do nothing but copy the next chunk from the float32 scratch, asynchronously.
 // S moves between registers and the request's state slot in an order of its own ([head][slice][row in lane][column]
 // [lane]), the same in both forms, so that the loads and stores of a decode step are coalesced.
-// Tokens are walked one by one whatever the step holds: the memory after a token does not depend on how the tokens
-// were cut into steps, and a token's output only in the order in which `lanes` parts are added.
+// Tokens are walked one by one whatever the step holds: how the tokens were cut into steps changes the memory after a
+// token and its output by rounding alone (the forms add a column's parts in orders of their own).
 //
 // A second kernel norms what the scan read out: RMS over groups of columns (a head, or all heads together), a
 // weight, a constant factor, and optionally a sigmoid gate from further columns of the product.

@@ -707,8 +707,8 @@ __global__ void __launch_bounds__(kGemvWarps * 32) moe_gemv_kernel(MoeGemmParams
 namespace {
 template <int FORM>
 int launch_moe_form(const MoeGemmParams& p, cudaStream_t stream) {
-  // 0: by size; 1: float arithmetic; 2: mma.sync tiles; 3: the few-rows form; 4: tcgen05 tiles.  The tcgen05 form is the
-  // fastest of all that it takes (us, gated / down product, 64 experts of 1,024 x 4,096 with 6 choices, tcgen05 |
+  // 0: by size; 1: float arithmetic; 2: mma.sync tiles; 3: the few-rows form; 4: tcgen05 tiles.  The tcgen05 form is
+  // faster than what a product ran on before it (us, gated / down product, 64 experts of 1,024 x 4,096 with 6 choices, tcgen05 |
   // mma.sync tiles | few rows: 1 token 43 / 22 | 81 / 33 | 62 / 29; 8 tokens 103 / 55 | 123 / 68 | 115 / 68; 64 tokens
   // 195 / 109 | 275 / 143 | 470 / 224; 2,048 tokens 282 / 185 | 881 / 520) but for one product: the first one of experts
   // without a gate on a few tokens.  A tcgen05 tile takes 256 features there, so a token's choices fill a handful of
@@ -716,7 +716,9 @@ int launch_moe_form(const MoeGemmParams& p, cudaStream_t stream) {
   // rows: 4 choices of 768 features 22.6 | 14.1, 16 choices 22.9 | 16.6; K = 4,096, 12 choices of 1,024 40.7 | 29.4).  It
   // wins while its blocks of 32 features run in one round (384 blocks; 576 took 28.7 against 23.1) and an expert's rows
   // are at most two of its passes (8 tokens that all choose the same experts 22 | 25, 12 tokens 26 | 27 to 52 | 44).
-  // The mma.sync tiles, and the few-rows form otherwise, serve hidden sizes below one K block of 64.
+  // The mma.sync tiles, and the few-rows form otherwise, serve hidden sizes below one K block of 64.  (Not taken: the down
+  // product of a few pairs whose weights lie in the L2 is faster in few rows, 4 pairs of 768 x 2,048 11.6 | 9.9, 8 pairs
+  // 11.7 | 13.8.)
   const bool few_blocks = FORM == kMoeUp && p.pairs <= kMoeFewRowPairs && p.pairs <= (int64_t)p.top * 2 * kGemvRows &&
                           p.pairs * ((p.n + kGemvFeatures - 1) / kGemvFeatures) <= 384;
   const bool tensor_ok = moe_gemm_takes_mma(p);
